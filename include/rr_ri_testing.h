@@ -68,6 +68,10 @@ int rr_test_half_transform(const double* Ct, int64_t nocc, const double* B, int6
 int rr_test_half_transform_time(const double* Ct, int64_t nocc, const double* B, int64_t naux, int64_t n, double* T,
                                 int32_t variant, int32_t reps, double* ms);
 
+/* Releases the resident digit planes of a store (rr_ri_create*), as if they had not fitted: its FP64 products then
+ * digitize ranges of aux rows on the fly.  *had = 1 when there were any. */
+int rr_test_drop_digit_planes(void* ri_handle, int32_t* had);
+
 /* Failure detection without a fault: one CTA of `threads` threads waits on an mbarrier that nothing
  * arrives on (and no bulk copy is in flight) through the bounded wait every TMA pipeline of the library
  * uses, with `spin_limit` polls (1 .. 4,194,304, the pipelines' own limit).  The wait expires, records

@@ -214,6 +214,7 @@ _SIGS = {
     "rr_test_mixed_exchange_delta": (ctypes.c_int, [_vp, _i64, _i64, _vp, _vp, _i64, _vp]),
     "rr_test_j_passes": (ctypes.c_int, [_vp, _i64, _i64, _vp, _vp, _vp]),
     "rr_test_j_passes_packed": (ctypes.c_int, [_vp, _i64, _i64, _vp, _vp, _vp, _vp]),
+    "rr_test_drop_digit_planes": (ctypes.c_int, [_vp, ctypes.POINTER(_i32)]),
     "rr_test_device_allocations": (ctypes.c_int64, []),
     "rr_test_half_transform": (ctypes.c_int, [_vp, _i64, _vp, _i64, _i64, _vp, _i32]),
     "rr_test_half_transform_time": (ctypes.c_int, [_vp, _i64, _vp, _i64, _i64, _vp, _i32, _i32, _vp]),

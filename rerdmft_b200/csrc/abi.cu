@@ -8,6 +8,7 @@
 
 #include "grouped.cuh"
 #include "mo_store.cuh"
+#include "oz_paths.cuh"
 
 namespace rr {
 extern thread_local std::string g_last_error;
@@ -52,8 +53,17 @@ void upload_tensor(rr::DevBuf<double>& dst, int64_t* pitch_out, const double* sr
   const int64_t pitch = rr::round_up(std::max<int64_t>(n2, 2), 32);
   *pitch_out = pitch;
   dst.alloc(static_cast<size_t>(std::max<int64_t>(naux * pitch, 32)));
-  RR_CUDA(cudaMemsetAsync(dst.p, 0, sizeof(double) * dst.n, s));
-  if (naux && n2)
+  // Only the padding is cleared, and rows without padding go in one linear copy: at n = 400, naux = 1600 the
+  // whole-buffer memset and the pitched copy took 2.4 ms of a store's creation (device source).
+  if (naux == 0 || n2 == 0) {
+    RR_CUDA(cudaMemsetAsync(dst.p, 0, sizeof(double) * dst.n, s));
+    return;
+  }
+  if (pitch > n2)
+    RR_CUDA(cudaMemset2DAsync(dst.p + n2, sizeof(double) * pitch, 0, sizeof(double) * (pitch - n2), naux, s));
+  if (pitch == n2)
+    RR_CUDA(cudaMemcpyAsync(dst.p, src, sizeof(double) * naux * n2, host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, s));
+  else
     RR_CUDA(cudaMemcpy2DAsync(dst.p, sizeof(double) * pitch, src, sizeof(double) * n2, sizeof(double) * n2, naux,
                               host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, s));
 }
@@ -140,6 +150,7 @@ int rr_ri_create(const double* B, int64_t naux, int64_t n, int32_t mem, rr_ri_ha
       RR_CUDA(cudaMemsetAsync(h->status.p, 0, 2 * sizeof(int), h->ctx.main));
       upload_tensor(h->B[0], &h->pitch[0], B, naux, n * n, mem == RR_MEM_HOST, h->ctx.main);
       rr::pack_for_j(h, 0, n, h->ctx.main);
+      rr::oz_prepare(h, 0, n, h->ctx.main);
       RR_CUDA(cudaStreamSynchronize(h->ctx.main));
     } catch (...) {
       h->ctx.destroy();
@@ -171,6 +182,8 @@ int rr_ri_create_4c(const double* B_LL, const double* B_SS, int64_t naux, int64_
       upload_tensor(h->B[1], &h->pitch[1], B_SS, naux, ns * ns, mem == RR_MEM_HOST, h->ctx.main);
       rr::pack_for_j(h, 0, nl, h->ctx.main);
       rr::pack_for_j(h, 1, ns, h->ctx.main);
+      rr::oz_prepare(h, 0, nl, h->ctx.main);
+      rr::oz_prepare(h, 1, ns, h->ctx.main);
       RR_CUDA(cudaStreamSynchronize(h->ctx.main));
     } catch (...) {
       h->ctx.destroy();
@@ -449,12 +462,9 @@ int rr_mo_build_nonrel(rr_ri_handle ri, const double* C, rr_mo_handle* out, cons
     auto* m = new_mo(0, s->naux, s->n);
     with_new_mo(out, m, [&] {
       cudaStream_t st = rr::call_stream(s, opts);
-      if (opts && opts->precision == RR_PREC_MIXED) {
-        rr::mo_build_nonrel_mixed(s, C, m, host_mem(opts), st);
-        rr::check_status(s, st);
-      } else {
-        rr::mo_build_nonrel(s, C, m, host_mem(opts), st);
-      }
+      if (opts && opts->precision == RR_PREC_MIXED) rr::mo_build_nonrel_mixed(s, C, m, host_mem(opts), st);
+      else rr::mo_build_nonrel(s, C, m, host_mem(opts), st);
+      rr::check_status(s, st);
       RR_CUDA(cudaStreamSynchronize(st));
     });
   });
@@ -473,7 +483,7 @@ int rr_mo_build_nonrel_into(rr_ri_handle ri, const double* C, rr_mo_handle mo, c
     if (mixed) rr::mo_build_nonrel_mixed(s, C, m, host_mem(opts), st);
     else rr::mo_build_nonrel(s, C, m, host_mem(opts), st);
     if (host_mem(opts) || (opts && opts->sync)) {
-      if (mixed) rr::check_status(s, st);
+      rr::check_status(s, st);
       RR_CUDA(cudaStreamSynchronize(st));
     }
   });
@@ -488,12 +498,9 @@ int rr_mo_build_ukb(rr_ri_handle ri4c, const double* c_ukb, int64_t n_total, rr_
     auto* m = new_mo(1, s->naux, n_total);
     with_new_mo(out, m, [&] {
       cudaStream_t st = rr::call_stream(s, opts);
-      if (opts && opts->precision == RR_PREC_MIXED) {
-        rr::mo_build_ukb_mixed(s, c_ukb, n_total, m, host_mem(opts), st);
-        rr::check_status(s, st);
-      } else {
-        rr::mo_build_ukb(s, c_ukb, n_total, m, host_mem(opts), st);
-      }
+      if (opts && opts->precision == RR_PREC_MIXED) rr::mo_build_ukb_mixed(s, c_ukb, n_total, m, host_mem(opts), st);
+      else rr::mo_build_ukb(s, c_ukb, n_total, m, host_mem(opts), st);
+      rr::check_status(s, st);
       RR_CUDA(cudaStreamSynchronize(st));
     });
   });

@@ -12,6 +12,7 @@
 #include <cstdlib>
 
 #include "ri_store.cuh"
+#include "oz_paths.cuh"
 
 namespace rr {
 
@@ -38,6 +39,7 @@ void coulomb_prep(rr_ri_store* h, const double* Dp, const double* Ct, int64_t no
                   cudaStream_t s, bool overlap);
 void coulomb_run(rr_ri_store* h, const double* tgam, int tseg, cudaStream_t s);
 void coulomb_join(rr_ri_store* h, cudaStream_t s);
+void coulomb_early(rr_ri_store* h, const double* Dp, double* J, cudaStream_t s, int ctas_per_sm);
 
 namespace {
 
@@ -105,6 +107,11 @@ void exchange_nonrel(rr_ri_store* h, const double* Ct, int64_t ldct, bool ct_tra
     if (K) RR_CUDA(cudaMemsetAsync(K, 0, sizeof(double) * n * n, s));
     if (Dp) coulomb_after_ht(h, Dp, Ct, 0, Jout, nullptr, 0, s);
     return;
+  }
+  if (K && !half_only && h->oz[0].ok && oz_worth(naux, n, nocc)) {
+    if (Dp) coulomb_early(h, Dp, Jout, s, 1);
+    if (oz_exchange_nonrel(h, Ct, ldct, ct_transposed, nocc, K, s)) return;
+    if (Dp) coulomb_join(h, s);  // no memory for the digit planes: the path below forms J again
   }
   h->T.ensure(static_cast<size_t>(naux * nocc * n));
   GemmDesc ht;

@@ -13,6 +13,7 @@
 #include <array>
 
 #include "ri_store.cuh"
+#include "oz_paths.cuh"
 
 namespace rr {
 
@@ -232,8 +233,14 @@ void two_electron_rel(rr_ri_store* h, const Flavours& fl, int64_t ntot, const do
       prof_mark(h, 3, s);
     }
   }
-  const bool fp64_k = !rb || !rb->mixed;
+  bool fp64_k = !rb || !rb->mixed;
   double* Gk = rb ? h->inc_k.p : G;  // where the FP64 blocks land
+  if (fp64_k && !energy_only && naux > 0 &&
+      oz_exchange_rel(h, fl.nf, fl.off.data(), fl.fs.data(), fl.tens.data(), ntot, Ct, r, rb ? nullptr : J, h->ctx.join, Gk,
+                      rb ? 1.0 : -1.0, s)) {
+    prof_mark(h, 3, s);
+    fp64_k = false;
+  }
   if (fp64_k && !energy_only) RR_CUDA(cudaMemsetAsync(Gk, 0, sizeof(double) * 2 * ntot * ntot, s));
   // T planes: flavour f occupies [Re (naux*r*fs) | Im (naux*r*fs)]; the off-diagonal blocks (f < u)
   // use Gauss's three products, with Re - Im of every flavour that is an f and Re + Im of every

@@ -419,7 +419,9 @@ bool j_pack_upper(const double* B, int64_t pitch, int64_t naux, int64_t n, DevBu
   RR_REQUIRE(n >= 1 && naux >= 1 && pitch >= n * n, RR_ERR_ARG, "j_pack_upper: bad shape");
   pitch_out = round_up(tri_len(n), 32);
   out.alloc(static_cast<size_t>(naux * pitch_out));
-  RR_CUDA(cudaMemsetAsync(out.p, 0, sizeof(double) * out.n, s));
+  // the kernel writes every triangle; the padding of the rows is cleared
+  if (pitch_out > tri_len(n))
+    RR_CUDA(cudaMemset2DAsync(out.p + tri_len(n), sizeof(double) * pitch_out, 0, sizeof(double) * (pitch_out - tri_len(n)), naux, s));
   DevBuf<int> asym(1);
   RR_CUDA(cudaMemsetAsync(asym.p, 0, sizeof(int), s));
   const int64_t ntile = (n + 31) / 32;

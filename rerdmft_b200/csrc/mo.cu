@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "mo_store.cuh"
+#include "oz_paths.cuh"
 
 namespace rr {
 
@@ -265,6 +266,7 @@ void mo_build_nonrel(rr_ri_store* ri, const double* C, rr_mo_store* m, bool host
   m->scratch.ensure(static_cast<size_t>(round_up(n * n, 32)));
   double* Cd = m->scratch.p;
   copy_in(Cd, C, n * n, host, s);
+  if (oz_mo_build_nonrel(ri, Cd, m, s)) return;
   const int64_t pc = chunk_rows(naux, n * n);
   m->T.ensure(static_cast<size_t>(pc * n * n));
   for (int64_t P0 = 0; P0 < naux; P0 += pc) {
@@ -297,6 +299,7 @@ void mo_build_ukb(rr_ri_store* ri, const double* c_ukb, int64_t nt, rr_mo_store*
   double* cd = m->scratch.p;
   double* Af = m->scratch.p + round_up(2 * nu * nt, 32);
   copy_in(cd, c_ukb, 2 * nu * nt, host, s);
+  if (oz_mo_build_ukb(ri, cd, nt, m, s)) return;
   const int64_t pc = chunk_rows(naux, 2 * nt * fsmax);
   m->T.ensure(static_cast<size_t>(pc * 2 * nt * fsmax));
   bool first = true;

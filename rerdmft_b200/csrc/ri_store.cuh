@@ -17,6 +17,17 @@ struct rr_ri_store {
   rr::DevBuf<double> Bpk[2];
   int64_t pitch_pk[2] = {0, 0};
   rr::DevBuf<int> status;   // device status word written by bounded waits
+  // Column scales, norms and digit planes of B[t] for the INT8 products (oz.cuh), filled with the store.  ok is
+  // false when B holds a NaN, an infinity or a value beyond 1e140, or n is too small for that path.  The
+  // planes (as large as B) are kept when they fit in a quarter of the free memory; otherwise the products
+  // digitize ranges of aux rows into their scratch.
+  struct {
+    bool ok = false;
+    rr::DevBuf<uint8_t> buf;  // all of the below
+    double *cscale = nullptr, *cnorm = nullptr, *pnorm = nullptr;
+    uint8_t* planes = nullptr;  // null: not kept
+  } oz[2];
+  rr::DevBuf<uint8_t> ozbuf;  // digit planes, exponents and partial sums of one call
   // Scratch, grown on demand and reused across calls.
   rr::DevBuf<double> mats;  // per-call matrices (inputs, outputs, intermediates)
   rr::DevBuf<double> T;     // half-transformed exchange intermediate

@@ -70,6 +70,24 @@ using rr::test_status;
 
 extern "C" {
 
+int rr_test_drop_digit_planes(void* ri_handle, int32_t* had) {
+  try {
+    rr::set_last_error("");
+    auto* h = static_cast<rr_ri_store*>(ri_handle);
+    RR_REQUIRE(h && had, RR_ERR_ARG, "rr_test_drop_digit_planes: null argument");
+    RR_CUDA(cudaDeviceSynchronize());
+    *had = 0;
+    for (auto& z : h->oz) {
+      if (z.planes) *had = 1;
+      z.planes = nullptr;
+    }
+    return RR_OK;
+  } catch (const rr::Error& e) {
+    rr::set_last_error(e.what());
+    return e.code;
+  }
+}
+
 int64_t rr_test_device_allocations(void) { return rr::device_allocations(); }
 
 int rr_test_half_transform(const double* Ct, int64_t nocc, const double* B, int64_t naux, int64_t n, double* T,
