@@ -72,6 +72,12 @@ int rr_test_half_transform_time(const double* Ct, int64_t nocc, const double* B,
  * digitize ranges of aux rows on the fly.  *had = 1 when there were any. */
 int rr_test_drop_digit_planes(void* ri_handle, int32_t* had);
 
+/* out = Y L^-dagger (times_l 0) or Y L (1) for M = L L^dagger (r x r) and n rows of Y (row-major, interleaved when cplx) by the
+ * one-launch factorisation of the occupied recovery; *ran = 0 when M does not fit shared memory (nothing is done),
+ * *status = 1 after a non-positive pivot. */
+int rr_test_chol_apply(const double* M, int64_t r, const double* Y, int64_t n, int32_t cplx, int32_t times_l, double* out,
+                       int32_t* ran, int32_t* status);
+
 /* Failure detection without a fault: one CTA of `threads` threads waits on an mbarrier that nothing
  * arrives on (and no bulk copy is in flight) through the bounded wait every TMA pipeline of the library
  * uses, with `spin_limit` polls (1 .. 4,194,304, the pipelines' own limit).  The wait expires, records

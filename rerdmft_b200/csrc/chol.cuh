@@ -121,4 +121,10 @@ __device__ __forceinline__ void chol_block_body(const double* M, int r, double* 
   }
 }
 
+// out = Y L^{-dagger}, or Y L with times_l, for M = L L^dagger (r x r, full) and the n rows of Y, on all SMs
+// (chol_apply.cu); near the identity Y M^{-1/2} or Y M^{1/2} instead.  status[0] |= 1 on a non-positive pivot.
+// Returns false, with nothing launched, when M and a CTA's rows do not fit shared memory.
+bool chol_apply(const double* M, int64_t r, const double* Y, int64_t n, bool cplx, bool times_l, double* out, int* status,
+                cudaStream_t s);
+
 }  // namespace rr

@@ -11,7 +11,8 @@
 //   2. W = Pi (NON_REL) or Pi P_eff Pi (weighted);
 //   3. an orthonormal basis Q of range(Pi) (rank r = trace Pi = number of eigenvalues > 1/2) by
 //      CholeskyQR2 of Pi G for a fixed pseudo-random G (deterministic), and F = Q for NON_REL or
-//      F = Q chol(Q^dagger P_eff Q) for the weighted case, so F F^dagger = W;
+//      F = Q chol(Q^dagger P_eff Q) for the weighted case, so F F^dagger = W (a Gram matrix near the
+//      identity is split symmetrically instead, chol_apply.cu);
 //   4. c_t = F^dagger X^dagger (r x n), the reference's c_t up to a unitary mixing of the occupied
 //      rows, which K is invariant to.
 // The Newton-Schulz residual read-back (which also yields trace Pi) is the only synchronisation.
@@ -106,13 +107,10 @@ __global__ void fill_test_matrix_kernel(double* G, int64_t count) {
   }
 }
 
-// SMEM selects the buffer at compile time, so the shared-memory variant addresses it with
-// shared-memory instructions (a pointer that may be either compiles to slower generic accesses).
-template <int PL, bool SMEM>
+template <int PL>
 __global__ void __launch_bounds__(CHOL_THREADS) chol_block_kernel(const double* M, int r, double* out,
                                                                   int want_inverse, int* status, double* gbuf) {
-  extern __shared__ double sm[];
-  chol_block_body<PL>(M, r, out, want_inverse, status, SMEM ? sm : gbuf);
+  chol_block_body<PL>(M, r, out, want_inverse, status, gbuf);
 }
 
 int blocks_for(int64_t n) { return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 1184))); }
@@ -142,9 +140,6 @@ void projector_ct(rr_ri_store* h, const double* A, const double* Pe, const doubl
   ar2.request(&PQ, n_eff * r * PL);
   ar2.request(&gw, 2 * r * (r | 1) * PL + r);
   ar2.commit();
-  // factor + inverse + pivots in shared memory when they fit, else in the global scratch gw
-  const size_t block_smem = sizeof(double) * (2 * r * (r | 1) * PL + r);
-  const bool chol_in_smem = block_smem <= 227 * 1024;
   if (cplx) fill_test_matrix_kernel<2><<<blocks_for(n_eff * r * 2), 256, 0, s>>>(G, n_eff * r);
   else fill_test_matrix_kernel<1><<<blocks_for(n_eff * r), 256, 0, s>>>(G, n_eff * r);
   RR_LAUNCH_CHECK();
@@ -153,14 +148,6 @@ void projector_ct(rr_ri_store* h, const double* A, const double* Pe, const doubl
   y.M = n_eff; y.N = r; y.K = n_eff;
   y.A = A; y.lda = n_eff; y.B = G; y.ldb = r; y.C = Y2; y.ldc = r;
   gemm(y, s, wk, wcap);
-  auto chol = [&](const double* mat, int inverse) {
-    const int sm = chol_in_smem ? static_cast<int>(block_smem) : 0;
-    auto k = cplx ? (chol_in_smem ? chol_block_kernel<2, true> : chol_block_kernel<2, false>)
-                  : (chol_in_smem ? chol_block_kernel<1, true> : chol_block_kernel<1, false>);
-    if (sm > 48 * 1024) RR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-    k<<<1, CHOL_THREADS, sm, s>>>(mat, static_cast<int>(r), Wt, inverse, h->status.p + 1, chol_in_smem ? nullptr : gw);
-    RR_LAUNCH_CHECK();
-  };
   GemmDesc gm;  // M = Y^dagger Y
   gm.cplx = cplx;
   gm.M = r; gm.N = r; gm.K = n_eff;
@@ -171,13 +158,23 @@ void projector_ct(rr_ri_store* h, const double* A, const double* Pe, const doubl
   yw.lda = r; yw.B = Wt; yw.ldb = r; yw.ldc = r;
   double* cur = Y2;
   double* nxt = Y3;
+  // cur <- cur L^{-dagger} (or cur L), M = L L^dagger: one launch while M fits shared memory (r <= 160 real, 112
+  // complex at 400 rows).  X2C, r = 80, 400 rows: 171 us for the one-CTA factor and inverse + 8 us for the product
+  // with it; larger r keep those two.
+  auto factor = [&](bool times_l) {
+    if (!chol_apply(M, r, cur, n_eff, cplx, times_l, nxt, h->status.p + 1, s)) {
+      auto k = cplx ? chol_block_kernel<2> : chol_block_kernel<1>;
+      k<<<1, CHOL_THREADS, 0, s>>>(M, static_cast<int>(r), Wt, times_l ? 0 : 1, h->status.p + 1, gw);
+      RR_LAUNCH_CHECK();
+      yw.A = cur; yw.C = nxt;
+      gemm(yw, s, wk, wcap);
+    }
+    std::swap(cur, nxt);
+  };
   for (int pass = 0; pass < 2; ++pass) {
     gm.A = cur; gm.B = cur;
     gemm(gm, s, wk, wcap);
-    chol(M, 1);
-    yw.A = cur; yw.C = nxt;
-    gemm(yw, s, wk, wcap);
-    std::swap(cur, nxt);
+    factor(false);
   }
   if (weighted) {  // F = Q chol(Q^dagger Pe Q): F F^dagger = Pi Pe Pi
     GemmDesc pq;
@@ -187,10 +184,7 @@ void projector_ct(rr_ri_store* h, const double* A, const double* Pe, const doubl
     gemm(pq, s, wk, wcap);
     gm.A = cur; gm.B = PQ;
     gemm(gm, s, wk, wcap);
-    chol(M, 0);
-    yw.A = cur; yw.C = nxt;
-    gemm(yw, s, wk, wcap);
-    std::swap(cur, nxt);
+    factor(true);
   }
   Y2 = cur;
   // c_t = F^dagger X^dagger  (r x n)

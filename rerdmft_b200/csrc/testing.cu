@@ -2,6 +2,7 @@
 // include/rr_ri_testing.h).  No reference counterpart.
 #include <algorithm>
 
+#include "chol.cuh"
 #include "ri_store.cuh"
 #include "gemm_f64.cuh"
 #include "tma_util.cuh"
@@ -81,6 +82,22 @@ int rr_test_drop_digit_planes(void* ri_handle, int32_t* had) {
       if (z.planes) *had = 1;
       z.planes = nullptr;
     }
+    return RR_OK;
+  } catch (const rr::Error& e) {
+    rr::set_last_error(e.what());
+    return e.code;
+  }
+}
+
+int rr_test_chol_apply(const double* M, int64_t r, const double* Y, int64_t n, int32_t cplx, int32_t times_l, double* out,
+                       int32_t* ran, int32_t* status) {
+  try {
+    rr::set_last_error("");
+    RR_REQUIRE(M && Y && out && ran && status && r >= 1 && n >= 1, RR_ERR_ARG, "rr_test_chol_apply: bad argument");
+    rr::DevBuf<int> st(1);
+    RR_CUDA(cudaMemset(st.p, 0, sizeof(int)));
+    *ran = rr::chol_apply(M, r, Y, n, cplx != 0, times_l != 0, out, st.p, nullptr) ? 1 : 0;
+    RR_CUDA(cudaMemcpy(status, st.p, sizeof(int), cudaMemcpyDeviceToHost));
     return RR_OK;
   } catch (const rr::Error& e) {
     rr::set_last_error(e.what());
