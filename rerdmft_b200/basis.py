@@ -23,6 +23,8 @@ from __future__ import annotations
 
 import math
 from dataclasses import dataclass, field
+from itertools import chain
+from operator import attrgetter, ne
 
 import numpy as np
 
@@ -312,15 +314,18 @@ def flatten(basis: list) -> dict:
     """Plain arrays of a BasisFunction list for the C ABI: center (n, 3), lxyz (n, 3) int32,
     prim_offset (n + 1) int64, exponents and coefficients (concatenated)."""
     n = len(basis)
-    center = np.array([[f.x, f.y, f.z] for f in basis], dtype=np.float64).reshape(n, 3)
-    lxyz = np.array([f.cartesian for f in basis], dtype=np.int32).reshape(n, 3)
+    center = np.fromiter(chain.from_iterable(map(attrgetter("x", "y", "z"), basis)), dtype=np.float64, count=3 * n).reshape(n, 3)
+    exponents, coefficients = [f.exponents for f in basis], [f.coefficients for f in basis]
+    count = np.fromiter(map(len, exponents), dtype=np.int64, count=n)
+    angular = [f.cartesian for f in basis]
+    if (n and count.min() == 0) or any(map(ne, map(len, coefficients), count.tolist())) or any(
+            map(ne, map(sum, angular), (f.l for f in basis))):
+        raise ValueError("flatten: inconsistent basis function")
+    lxyz = np.array(list(chain.from_iterable(angular)), dtype=np.int32).reshape(n, 3)
     off = np.zeros(n + 1, dtype=np.int64)
-    off[1:] = np.cumsum([len(f.exponents) for f in basis])
-    exps = np.array([e for f in basis for e in f.exponents], dtype=np.float64)
-    coefs = np.array([c for f in basis for c in f.coefficients], dtype=np.float64)
-    for f in basis:
-        if sum(f.cartesian) != f.l or len(f.exponents) != len(f.coefficients) or not f.exponents:
-            raise ValueError("flatten: inconsistent basis function")
+    np.cumsum(count, out=off[1:])
+    exps = np.array(list(chain.from_iterable(exponents)), dtype=np.float64)
+    coefs = np.array(list(chain.from_iterable(coefficients)), dtype=np.float64)
     return dict(center=np.ascontiguousarray(center), lxyz=np.ascontiguousarray(lxyz), prim_offset=off,
                 exponents=exps, coefficients=coefs)
 

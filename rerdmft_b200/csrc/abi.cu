@@ -71,7 +71,7 @@ void upload_tensor(rr::DevBuf<double>& dst, int64_t* pitch_out, const double* sr
 rr_mo_store* new_mo(int cplx, int64_t naux, int64_t n) {
   auto* m = new rr_mo_store();
   try {
-    m->ctx.init(nullptr);
+    m->ctx.init(nullptr, false);
   } catch (...) {
     delete m;
     throw;

@@ -857,7 +857,7 @@ int rr_orbopt_create(rr_mo_handle m, const double* h, const double* occupations,
         RR_REQUIRE(pair_of[i] >= 0 && pair_of[i] < d, RR_ERR_ARG, "rr_orbopt_create: pair_of out of range");
     auto* o = new rr_orbopt_store();
     try {
-      o->ctx.init(nullptr);
+      o->ctx.init(nullptr, false);
       o->cplx = cplx;
       o->PL = PL;
       o->n = n;

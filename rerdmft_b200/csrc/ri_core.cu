@@ -3,6 +3,9 @@
 #include <algorithm>
 #include <atomic>
 #include <complex>
+#include <map>
+#include <mutex>
+#include <unordered_map>
 
 #include "ri_store.cuh"
 
@@ -18,6 +21,109 @@ int64_t launches() { return g_launches.load(std::memory_order_relaxed); }
 static std::atomic<int64_t> g_device_allocs{0};
 void count_device_alloc() { g_device_allocs.fetch_add(1, std::memory_order_relaxed); }
 int64_t device_allocations() { return g_device_allocs.load(std::memory_order_relaxed); }
+
+namespace {
+
+// Blocks handed out and blocks kept, per device.  Objects with large tensors are made and dropped in a user's loop
+// (one MO tensor per rotation): each cudaMalloc and cudaFree of their buffers takes 300 - 500 us.
+struct DevicePool {
+  struct Live {
+    size_t bytes;
+    int dev;
+  };
+  std::mutex mu;
+  std::unordered_map<void*, Live> live;
+  std::multimap<size_t, void*> kept[kMaxDevices];
+  size_t kept_bytes[kMaxDevices] = {}, limit[kMaxDevices] = {};
+  int64_t live_count[kMaxDevices] = {};
+
+  void trim(int dev) {  // mu held
+    for (auto& b : kept[dev]) cudaFree(b.second);
+    kept[dev].clear();
+    kept_bytes[dev] = 0;
+  }
+};
+constexpr size_t kPoolShare = 64;  // of the device's memory, one part (2.8 GB of 180)
+DevicePool& pool() {
+  static DevicePool* p = new DevicePool();  // never destroyed: handles may outlive static destructors
+  return *p;
+}
+
+}  // namespace
+
+void* device_alloc(size_t bytes) {
+  const int dev = current_device();
+  const size_t unit = bytes >= (size_t{1} << 20) ? size_t{1} << 20 : 512, size = (bytes + unit - 1) / unit * unit;
+  DevicePool& pl = pool();
+  const bool pooled = dev >= 0 && dev < kMaxDevices;
+  void* p = nullptr;
+  if (pooled) {
+    std::lock_guard<std::mutex> lock(pl.mu);
+    auto it = pl.kept[dev].lower_bound(size);
+    if (it != pl.kept[dev].end() && it->first <= size + size / 8) {
+      p = it->second;
+      pl.live[p] = {it->first, dev};
+      pl.kept_bytes[dev] -= it->first;
+      pl.kept[dev].erase(it);
+      ++pl.live_count[dev];
+      return p;
+    }
+  }
+  cudaError_t e = cudaMalloc(&p, size);
+  if (e == cudaErrorMemoryAllocation && pooled) {
+    cudaGetLastError();
+    {
+      std::lock_guard<std::mutex> lock(pl.mu);
+      pl.trim(dev);
+    }
+    e = cudaMalloc(&p, size);
+  }
+  if (e != cudaSuccess) throw Error(RR_ERR_CUDA, std::string("cudaMalloc failed: ") + cudaGetErrorString(e));
+  if (pooled) {
+    std::lock_guard<std::mutex> lock(pl.mu);
+    pl.live[p] = {size, dev};
+    ++pl.live_count[dev];
+  }
+  return p;
+}
+
+void device_free(void* p) noexcept {
+  DevicePool& pl = pool();
+  DevicePool::Live b{0, -1};
+  {
+    std::lock_guard<std::mutex> lock(pl.mu);
+    auto it = pl.live.find(p);
+    if (it != pl.live.end()) {
+      b = it->second;
+      pl.live.erase(it);
+    }
+  }
+  if (b.dev < 0) {
+    cudaFree(p);
+    return;
+  }
+  // cudaFree's wait, on the block's device
+  int cur = b.dev;
+  bool ok = cudaGetDevice(&cur) == cudaSuccess;
+  if (ok && cur != b.dev) ok = cudaSetDevice(b.dev) == cudaSuccess;
+  ok = ok && cudaDeviceSynchronize() == cudaSuccess;
+  {
+    std::lock_guard<std::mutex> lock(pl.mu);
+    if (ok && pl.limit[b.dev] == 0) {
+      size_t free_b = 0, total_b = 0;
+      if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) pl.limit[b.dev] = total_b / kPoolShare;
+    }
+    const bool last = --pl.live_count[b.dev] == 0;
+    if (ok && !last && pl.kept_bytes[b.dev] + b.bytes <= pl.limit[b.dev]) {
+      pl.kept[b.dev].emplace(b.bytes, p);
+      pl.kept_bytes[b.dev] += b.bytes;
+    } else {
+      cudaFree(p);
+    }
+    if (last) pl.trim(b.dev);
+  }
+  if (cur != b.dev) cudaSetDevice(cur);
+}
 
 int current_device() {
   int dev = 0;
@@ -35,7 +141,7 @@ int sm_count_current() {
   return sms;
 }
 
-void Context::init(cudaStream_t user_stream) {
+void Context::init(cudaStream_t user_stream, bool fock) {
   RR_CUDA(cudaGetDevice(&device));
   if (user_stream) {
     main = user_stream;
@@ -44,6 +150,7 @@ void Context::init(cudaStream_t user_stream) {
     RR_CUDA(cudaStreamCreateWithFlags(&main, cudaStreamNonBlocking));
     own_main = true;
   }
+  if (!fock) return;
   // The side stream carries the bandwidth-bound Coulomb passes that run alongside compute-bound
   // GEMMs on the main stream; its higher priority lets their CTAs be dispatched as GEMM CTAs retire.
   int lo = 0, hi = 0;
@@ -55,7 +162,12 @@ void Context::init(cudaStream_t user_stream) {
   for (auto& e : upl) RR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   RR_CUDA(cudaStreamCreateWithFlags(&pipe_stream, cudaStreamNonBlocking));
   for (auto& e : pipe_ev) RR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  RR_SOLVER(cusolverDnCreate(&solver));
+  solver_handle();
+}
+
+cusolverDnHandle_t Context::solver_handle() {
+  if (!solver) RR_SOLVER(cusolverDnCreate(&solver));
+  return solver;
 }
 
 void Context::destroy() {
@@ -177,7 +289,7 @@ void fock_combine(double* F, const double* h, const double* J, const double* K, 
 
 void eigh_sym_ctx(Context& c, double* a, int64_t n, double* w, cudaStream_t s) {
   if (n == 0) return;
-  RR_SOLVER(cusolverDnSetStream(c.solver, s));
+  RR_SOLVER(cusolverDnSetStream(c.solver_handle(), s));
   int lwork = 0;
   RR_SOLVER(cusolverDnDsyevd_bufferSize(c.solver, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER, static_cast<int>(n),
                                         a, static_cast<int>(n), w, &lwork));
@@ -189,7 +301,7 @@ void eigh_sym_ctx(Context& c, double* a, int64_t n, double* w, cudaStream_t s) {
 
 void eigh_herm_ctx(Context& c, double* a, int64_t n, double* w, cudaStream_t s) {
   if (n == 0) return;
-  RR_SOLVER(cusolverDnSetStream(c.solver, s));
+  RR_SOLVER(cusolverDnSetStream(c.solver_handle(), s));
   int lwork = 0;
   auto* az = reinterpret_cast<cuDoubleComplex*>(a);
   RR_SOLVER(cusolverDnZheevd_bufferSize(c.solver, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER, static_cast<int>(n),

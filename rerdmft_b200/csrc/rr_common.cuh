@@ -59,7 +59,15 @@ void count_launch();
 // Counts the device allocations the library makes (DevBuf::alloc); read by a test hook.
 void count_device_alloc();
 
-// Owning device allocation (cudaMalloc/cudaFree), move-only.
+// Device memory behind DevBuf (ri_core.cu).  device_free keeps a released block for a later device_alloc of about its
+// size on the same device, up to kPoolShare of the device's memory in all; a block that does not fit that
+// bound goes back to the driver at once, all of them do when the last DevBuf of the device is released or an allocation
+// fails.  Like cudaFree, device_free returns only after the work queued on the device is done, so a block never
+// changes hands while a stream or a thread still uses it.
+void* device_alloc(size_t bytes);
+void device_free(void* p) noexcept;
+
+// Owning device allocation, move-only.
 template <typename T>
 struct DevBuf {
   T* p = nullptr;
@@ -77,7 +85,7 @@ struct DevBuf {
   void alloc(size_t count) {
     release();
     if (count) {
-      RR_CUDA(cudaMalloc(&p, count * sizeof(T)));
+      p = static_cast<T*>(device_alloc(count * sizeof(T)));
       count_device_alloc();
     }
     n = count;
@@ -85,7 +93,7 @@ struct DevBuf {
   // Grow-only: keeps the allocation when it is already large enough.
   void ensure(size_t count) { if (count > n) alloc(count); }
   void release() {
-    if (p) cudaFree(p);
+    if (p) device_free(p);
     p = nullptr;
     n = 0;
   }
@@ -108,7 +116,11 @@ struct Context {
   cusolverDnHandle_t solver = nullptr;
   DevBuf<double> solver_work;
   DevBuf<int> solver_info;
-  void init(cudaStream_t user_stream);
+  // fock: with the side and pipe streams, the events and the cuSOLVER handle of the Fock builds and SCF loops.
+  // Contexts of MO tensors and orbital optimisers run on the main stream alone, and most never solve an eigenproblem:
+  // solver_handle() makes theirs on first use (cusolverDnCreate and Destroy take 2.7 + 2.4 ms).
+  void init(cudaStream_t user_stream, bool fock = true);
+  cusolverDnHandle_t solver_handle();
   void destroy();
   void set_stream(cudaStream_t s);
 };

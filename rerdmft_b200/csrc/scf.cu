@@ -537,7 +537,7 @@ void ritz_bounds(rr_ri_store* h, const double* F, int64_t n, bool cplx, double* 
   t.mirror = 1;
   gemm(t, s, h->work.p, static_cast<int64_t>(h->work.n));
   auto& c = h->ctx;
-  RR_SOLVER(cusolverDnSetStream(c.solver, s));
+  RR_SOLVER(cusolverDnSetStream(c.solver_handle(), s));
   c.solver_info.ensure(1);
   int lwork = 0;
   if (cplx) {
