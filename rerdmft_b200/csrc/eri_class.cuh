@@ -4,6 +4,7 @@
 #pragma once
 
 #include <cmath>
+#include <utility>
 
 #include "ri_store.cuh"
 
@@ -75,6 +76,33 @@ __host__ __device__ constexpr int rix(int t, int u, int v) {
   return (t + u + v) * (t + u + v + 1) * (t + u + v + 2) / 6 + (u + v) * (u + v + 1) / 2 + v;
 }
 
+__host__ __device__ constexpr int n_herm(int l) { return (l + 1) * (l + 2) * (l + 3) / 6; }
+
+// (t, u, v) of a flat Hermite index (the inverse of rix).
+struct Herm {
+  int t, u, v;
+};
+__host__ __device__ constexpr Herm herm_of(int i) {
+  int s = 0;
+  while (n_herm(s) <= i) ++s;
+  const int e = i - s * (s + 1) * (s + 2) / 6;
+  int m = 0;
+  while ((m + 1) * (m + 2) / 2 <= e) ++m;
+  const int v = e - m * (m + 1) / 2;
+  return Herm{s - m, m - v, v};
+}
+
+// f(std::integral_constant<int, 0>()) ... f(N - 1): the loops over Hermite and component indices.  (Unroll pragmas on
+// their nested triangular form left the tables in local memory, addressed at run time, from three indices on.)
+template <class F, int... I>
+__device__ __forceinline__ void static_for_seq(F&& f, std::integer_sequence<int, I...>) {
+  (f(std::integral_constant<int, I>()), ...);
+}
+template <int N, class F>
+__device__ __forceinline__ void static_for(F&& f) {
+  static_for_seq(static_cast<F&&>(f), std::make_integer_sequence<int, N>());
+}
+
 struct ClassArgs {
   const DShell* sh;
   const double* ex;
@@ -95,106 +123,102 @@ struct ClassArgs {
 template <int LA, int LB>
 __device__ __forceinline__ void e_fixed(double (&E)[LA + 1][LB + 1][LA + LB + 1], double inv2p, double xpa,
                                        double xpb) {
-#pragma unroll
-  for (int i = 0; i <= LA; ++i)
-#pragma unroll
-    for (int j = 0; j <= LB; ++j)
-#pragma unroll
-      for (int t = 0; t <= LA + LB; ++t) {
-        double v;
-        if (i == 0 && j == 0) {
-          v = t == 0 ? 1.0 : 0.0;
-        } else if (t > i + j) {
-          v = 0.0;
-        } else if (i > 0) {
-          v = xpa * E[i - 1][j][t];
-          if (t > 0) v += inv2p * E[i - 1][j][t - 1];
-          if (t + 1 <= i + j - 1) v += (t + 1) * E[i - 1][j][t + 1];
-        } else {
-          v = xpb * E[i][j - 1][t];
-          if (t > 0) v += inv2p * E[i][j - 1][t - 1];
-          if (t + 1 <= i + j - 1) v += (t + 1) * E[i][j - 1][t + 1];
-        }
-        E[i][j][t] = v;
-      }
-}
-
-__host__ __device__ constexpr int n_herm(int l) { return (l + 1) * (l + 2) * (l + 3) / 6; }
-
-// acc[(ia NB + ib) STRIDE] += w (a b | component IC of c) for one primitive triple, from the E tables of the
-// pair, the Hermite Coulomb integrals R and the aux factor's Hermite coefficients Ec; every index is a
-// compile-time constant.
-template <int LA, int LB, int LC, int IC, int STRIDE>
-__device__ __forceinline__ void accum_comp(double* acc, const double (&E)[3][LA + 1][LB + 1][LA + LB + 1],
-                                           const double (&R)[n_herm(LA + LB + LC)],
-                                           const double (&Ec)[LC + 1][LC + 1], double w) {
-  constexpr int NA = Cart<LA>::N, NB = Cart<LB>::N, LAB = LA + LB;
-  constexpr int cx = cart_comp(LC, IC, 0), cy = cart_comp(LC, IC, 1), cz = cart_comp(LC, IC, 2);
-  double G[n_herm(LAB)];
-#pragma unroll
-  for (int sl = 0; sl <= LAB; ++sl)
-#pragma unroll
-    for (int m = 0; m <= sl; ++m)
-#pragma unroll
-      for (int v = 0; v <= m; ++v) {
-        const int u = m - v, t = sl - m;
-        double g = 0.0;
-#pragma unroll
-        for (int tau = cx & 1; tau <= cx; tau += 2)
-#pragma unroll
-          for (int nu = cy & 1; nu <= cy; nu += 2)
-#pragma unroll
-            for (int phi = cz & 1; phi <= cz; phi += 2) {
-              const double ec = Ec[cx][tau] * Ec[cy][nu] * Ec[cz][phi];
-              const double r = R[rix(t + tau, u + nu, v + phi)];
-              g += ((tau + nu + phi) & 1) ? -ec * r : ec * r;
-            }
-        G[rix(t, u, v)] = g;
-      }
-#pragma unroll
-  for (int ia = 0; ia < NA; ++ia)
-#pragma unroll
-    for (int ib = 0; ib < NB; ++ib) {
-      const int ax = cart_comp(LA, ia, 0), ay = cart_comp(LA, ia, 1), az = cart_comp(LA, ia, 2);
-      const int bx = cart_comp(LB, ib, 0), by = cart_comp(LB, ib, 1), bz = cart_comp(LB, ib, 2);
-      double val = 0.0;
-#pragma unroll
-      for (int t = 0; t <= ax + bx; ++t)
-#pragma unroll
-        for (int u = 0; u <= ay + by; ++u)
-#pragma unroll
-          for (int v = 0; v <= az + bz; ++v)
-            val += E[0][ax][bx][t] * E[1][ay][by][u] * E[2][az][bz][v] * G[rix(t, u, v)];
-      acc[(ia * NB + ib) * STRIDE] += w * val;
+  static_for<(LA + 1) * (LB + 1) * (LA + LB + 1)>([&](auto c) {
+    constexpr int f = decltype(c)::value, t = f % (LA + LB + 1), j = f / (LA + LB + 1) % (LB + 1), i = f / (LA + LB + 1) / (LB + 1);
+    double v = 0.0;
+    if constexpr (i == 0 && j == 0) {
+      v = t == 0 ? 1.0 : 0.0;
+    } else if constexpr (t <= i + j) {
+      constexpr int si = i > 0 ? i - 1 : i, sj = i > 0 ? j : j - 1;
+      v = (i > 0 ? xpa : xpb) * E[si][sj][t];
+      if constexpr (t > 0) v += inv2p * E[si][sj][t - 1];
+      if constexpr (t + 1 <= i + j - 1) v += (t + 1) * E[si][sj][t + 1];
     }
+    E[i][j][t] = v;
+  });
 }
 
-// Every component, acc[(ia NB + ib) NC + ic].
+// G[tuv]: the Hermite Coulomb integrals R contracted with component IC of the aux factor (Hermite coefficients Ec);
+// every index is a compile-time constant.
+template <int LAB, int LC, int IC>
+__device__ __forceinline__ void herm_comp(double (&G)[n_herm(LAB)], const double (&R)[n_herm(LAB + LC)],
+                                          const double (&Ec)[LC + 1][LC + 1]) {
+  constexpr int cx = cart_comp(LC, IC, 0), cy = cart_comp(LC, IC, 1), cz = cart_comp(LC, IC, 2);
+  constexpr int nx = cx / 2 + 1, ny = cy / 2 + 1, nz = cz / 2 + 1;  // tau = cx, cx - 2, ... and so on
+  static_for<n_herm(LAB)>([&](auto c) {
+    constexpr Herm h = herm_of(decltype(c)::value);
+    double g = 0.0;
+    static_for<nx * ny * nz>([&](auto k) {
+      constexpr int i = decltype(k)::value;
+      constexpr int tau = (cx & 1) + 2 * (i / (ny * nz)), nu = (cy & 1) + 2 * (i / nz % ny), phi = (cz & 1) + 2 * (i % nz);
+      const double ec = Ec[cx][tau] * Ec[cy][nu] * Ec[cz][phi];
+      const double r = R[rix(h.t + tau, h.u + nu, h.v + phi)];
+      g += ((tau + nu + phi) & 1) ? -ec * r : ec * r;
+    });
+    G[decltype(c)::value] = g;
+  });
+}
+
+// The thread's one component `ic` (uniform over nearly every warp).
+template <int LAB, int LC, int IC>
+__device__ __forceinline__ void herm_dispatch(int ic, double (&G)[n_herm(LAB)], const double (&R)[n_herm(LAB + LC)],
+                                              const double (&Ec)[LC + 1][LC + 1]) {
+  if constexpr (IC < Cart<LC>::N) {
+    if (ic == IC) herm_comp<LAB, LC, IC>(G, R, Ec);
+    else herm_dispatch<LAB, LC, IC + 1>(ic, G, R, Ec);
+  }
+}
+
+// acc[(ia NB + ib) STRIDE] += w sum_tuv E_t E_u E_v G_tuv for every component pair, one dimension after the other.
+template <int LA, int LB, int STRIDE>
+__device__ __forceinline__ void bra_comps(double* acc, const double (&E)[3][LA + 1][LB + 1][LA + LB + 1],
+                                          const double (&G)[n_herm(LA + LB)], double w) {
+  constexpr int NA = Cart<LA>::N, NB = Cart<LB>::N;
+  static_for<NA * NB>([&](auto c) {
+    constexpr int ia = decltype(c)::value / NB, ib = decltype(c)::value % NB;
+    constexpr int ax = cart_comp(LA, ia, 0), ay = cart_comp(LA, ia, 1), az = cart_comp(LA, ia, 2);
+    constexpr int bx = cart_comp(LB, ib, 0), by = cart_comp(LB, ib, 1), bz = cart_comp(LB, ib, 2);
+    double val = 0.0;
+    static_for<ax + bx + 1>([&](auto ct) {
+      constexpr int t = decltype(ct)::value;
+      double vt = 0.0;
+      static_for<ay + by + 1>([&](auto cu) {
+        constexpr int u = decltype(cu)::value;
+        double vu = 0.0;
+        static_for<az + bz + 1>([&](auto cv) {
+          constexpr int v = decltype(cv)::value;
+          const double g = G[rix(t, u, v)];
+          if constexpr (v == 0) vu = E[2][az][bz][0] * g;
+          else vu = fma(E[2][az][bz][v], g, vu);
+        });
+        if constexpr (u == 0) vt = E[1][ay][by][0] * vu;
+        else vt = fma(E[1][ay][by][u], vu, vt);
+      });
+      if constexpr (t == 0) val = E[0][ax][bx][0] * vt;
+      else val = fma(E[0][ax][bx][t], vt, val);
+    });
+    acc[decltype(c)::value * STRIDE] = fma(w, val, acc[decltype(c)::value * STRIDE]);
+  });
+}
+
+// Every aux component, acc[(ia NB + ib) NC + ic].
 template <int LA, int LB, int LC, int IC>
 __device__ __forceinline__ void comp_all(double* acc, const double (&E)[3][LA + 1][LB + 1][LA + LB + 1],
                                          const double (&R)[n_herm(LA + LB + LC)],
                                          const double (&Ec)[LC + 1][LC + 1], double w) {
   if constexpr (IC < Cart<LC>::N) {
-    accum_comp<LA, LB, LC, IC, Cart<LC>::N>(acc + IC, E, R, Ec, w);
+    double G[n_herm(LA + LB)];
+    herm_comp<LA + LB, LC, IC>(G, R, Ec);
+    bra_comps<LA, LB, Cart<LC>::N>(acc + IC, E, G, w);
     comp_all<LA, LB, LC, IC + 1>(acc, E, R, Ec, w);
   }
 }
 
-// The thread's one component `ic`, acc[ia NB + ib].
-template <int LA, int LB, int LC, int IC>
-__device__ __forceinline__ void comp_dispatch(int ic, double* acc, const double (&E)[3][LA + 1][LB + 1][LA + LB + 1],
-                                              const double (&R)[n_herm(LA + LB + LC)],
-                                              const double (&Ec)[LC + 1][LC + 1], double w) {
-  if constexpr (IC < Cart<LC>::N) {
-    if (ic == IC)
-      accum_comp<LA, LB, LC, IC, 1>(acc, E, R, Ec, w);
-    else
-      comp_dispatch<LA, LB, LC, IC + 1>(ic, acc, E, R, Ec, w);
-  }
-}
-
-// SPLIT: one thread per (pair, aux shell, aux component) for the classes with many outputs; the component
-// is selected among compile-time branches, so every table index stays static.
+// SPLIT: one thread per (pair, aux shell, aux component) for the classes with many outputs; only the contraction of R
+// with the component is selected among compile-time branches (every table index stays static), the bra side is
+// common to all of them.
+//
+// Primitive pairs whose K_AB underflows to zero are skipped: every term they would add is a zero.
 template <int LA, int LB, int LC, bool SPLIT>
 __global__ void __launch_bounds__(128) eri_class_kernel(ClassArgs a) {
   constexpr int NA = Cart<LA>::N, NB = Cart<LB>::N, NC = Cart<LC>::N, NCA = SPLIT ? 1 : NC;
@@ -222,9 +246,14 @@ __global__ void __launch_bounds__(128) eri_class_kernel(ClassArgs a) {
         const double p = al + be, ip = 1.0 / p;
         const double P[3] = {(al * A.x + be * B.x) * ip, (al * A.y + be * B.y) * ip, (al * A.z + be * B.z) * ip};
         const double K = exp(-al * be * ip * ab2);
+        if (K == 0.0) continue;
+        // from L = 5 on the pair's E tables are made after R is used up: both do not fit the registers together
+        constexpr bool E_LATE = SPLIT && L >= 5;
         double E[3][LA + 1][LB + 1][LAB + 1];
+        if constexpr (!E_LATE) {
 #pragma unroll
-        for (int d = 0; d < 3; ++d) e_fixed<LA, LB>(E[d], 0.5 * ip, -be * ip * ab[d], al * ip * ab[d]);
+          for (int d = 0; d < 3; ++d) e_fixed<LA, LB>(E[d], 0.5 * ip, -be * ip * ab[d], al * ip * ab[d]);
+        }
         for (int k = 0; k < C.nprim; ++k) {
           const double ga = a.ex[C.prim0 + k], cC = a.co[C.prim0 + k];
           const double alpha = p * ga / (p + ga);
@@ -237,49 +266,50 @@ __global__ void __launch_bounds__(128) eri_class_kernel(ClassArgs a) {
           for (int n = 1; n <= L; ++n) pw[n] = pw[n - 1] * (-2.0 * alpha);
           double R[NR];
           R[0] = pw[L] * F[L];
-#pragma unroll
-          for (int n = L - 1; n >= 0; --n) {
-#pragma unroll
-            for (int sl = L - n; sl >= 1; --sl)
-#pragma unroll
-              for (int m = 0; m <= sl; ++m)
-#pragma unroll
-                for (int v = 0; v <= m; ++v) {
-                  const int u = m - v, t = sl - m;
-                  double val;
-                  if (t > 0) {
-                    val = X * R[rix(t - 1, u, v)];
-                    if (t > 1) val += (t - 1) * R[rix(t - 2, u, v)];
-                  } else if (u > 0) {
-                    val = Y * R[rix(t, u - 1, v)];
-                    if (u > 1) val += (u - 1) * R[rix(t, u - 2, v)];
-                  } else {
-                    val = Z * R[rix(t, u, v - 1)];
-                    if (v > 1) val += (v - 1) * R[rix(t, u, v - 2)];
-                  }
-                  R[rix(t, u, v)] = val;
-                }
+          // step n: levels L - n .. 1 in place, each from the two below it of step n + 1
+          static_for<L>([&](auto cn) {
+            constexpr int n = L - 1 - decltype(cn)::value, top = n_herm(L - n) - 1;
+            static_for<top>([&](auto ce) {
+              constexpr int e = top - decltype(ce)::value;
+              constexpr Herm h = herm_of(e);
+              double val;
+              if constexpr (h.t > 0) {
+                val = X * R[rix(h.t - 1, h.u, h.v)];
+                if constexpr (h.t > 1) val += (h.t - 1) * R[rix(h.t - 2, h.u, h.v)];
+              } else if constexpr (h.u > 0) {
+                val = Y * R[rix(h.t, h.u - 1, h.v)];
+                if constexpr (h.u > 1) val += (h.u - 1) * R[rix(h.t, h.u - 2, h.v)];
+              } else {
+                val = Z * R[rix(h.t, h.u, h.v - 1)];
+                if constexpr (h.v > 1) val += (h.v - 1) * R[rix(h.t, h.u, h.v - 2)];
+              }
+              R[e] = val;
+            });
             R[0] = pw[n] * F[n];
-          }
+          });
           // single-centre Hermite coefficients of the aux factor, Ec[i][t] (t = i, i - 2, ...)
           double Ec[LC + 1][LC + 1];
           const double inv2q = 0.5 / ga;
-#pragma unroll
-          for (int ii = 0; ii <= LC; ++ii)
-#pragma unroll
-            for (int t = 0; t <= LC; ++t) {
-              double v = 0.0;
-              if (ii == 0) {
-                v = t == 0 ? 1.0 : 0.0;
-              } else {
-                if (t > 0) v += inv2q * Ec[ii - 1][t - 1];
-                if (t + 1 <= LC) v += (t + 1) * Ec[ii - 1][t + 1];
-              }
-              Ec[ii][t] = v;
+          static_for<(LC + 1) * (LC + 1)>([&](auto c) {
+            constexpr int ii = decltype(c)::value / (LC + 1), t = decltype(c)::value % (LC + 1);
+            double v = 0.0;
+            if constexpr (ii == 0) {
+              v = t == 0 ? 1.0 : 0.0;
+            } else {
+              if constexpr (t > 0) v += inv2q * Ec[ii - 1][t - 1];
+              if constexpr (t + 1 <= LC) v += (t + 1) * Ec[ii - 1][t + 1];
             }
+            Ec[ii][t] = v;
+          });
           const double w = cA * cB * cC * two_pi25 / (p * ga * sqrt(p + ga)) * K;
           if constexpr (SPLIT) {
-            comp_dispatch<LA, LB, LC, 0>(icsel, acc, E, R, Ec, w);
+            double G[n_herm(LAB)];
+            herm_dispatch<LAB, LC, 0>(icsel, G, R, Ec);
+            if constexpr (E_LATE) {
+#pragma unroll
+              for (int d = 0; d < 3; ++d) e_fixed<LA, LB>(E[d], 0.5 * ip, -be * ip * ab[d], al * ip * ab[d]);
+            }
+            bra_comps<LA, LB, 1>(acc, E, G, w);
           } else {
             comp_all<LA, LB, LC, 0>(acc, E, R, Ec, w);
           }
@@ -327,9 +357,12 @@ __global__ void __launch_bounds__(128) eri_class_kernel(ClassArgs a) {
 
 // Launch of one class kernel (grid-stride, 8 waves of the occupancy at most).  The classes with such a
 // kernel (l_A >= l_B, aux l <= 3): one thread per item for the s and p pairs with aux s .. f, (pp| s, p)
-// and (ds| s, p); one thread per aux component for (pp| d, f), (ds| d, f) and (dp| s, p, d).  The rest
-// take the warp kernel of integrals.cu: (dd| ...), l >= 3, and (dp| f), whose template alone compiled for
-// 9 minutes (1.35 of the 12.2 ms of the (H2O)_8 / cc-pVDZ raw tensor ran there before the dp templates).
+// and (ds| s, p); one thread per aux component for (pp| d, f), (ds| d, f), (dp| ...), (dd| ...) and (fs| ...).  The
+// rest (aux l >= 4, the other l >= 3 pairs) take the warp kernel of integrals.cu, which serialises the table set-up of
+// a primitive triple on single lanes: for the raw tensor of (H2O)_8 / cc-pVDZ (dp|f) takes 131 us here against 1331
+// there, the four (dd| ...) classes 230 against 1540.
+//
+// Bound: FP64 latency (about 30 % of the FP64 pipe, 7 - 17 % of the warp slots at 100 - 255 registers).
 template <int LA, int LB, int LC, bool SPLIT>
 void launch_class(const ClassArgs& a, cudaStream_t s) {
   auto kern = eri_class_kernel<LA, LB, LC, SPLIT>;
@@ -350,6 +383,8 @@ bool launch_class_sp(int la, int lb, int lc, const ClassArgs& a, cudaStream_t s)
 bool launch_class_split(int la, int lb, int lc, const ClassArgs& a, cudaStream_t s);  // eri_class_split.cu
 bool launch_class_dp01(int la, int lb, int lc, const ClassArgs& a, cudaStream_t s);   // eri_class_dp01.cu
 bool launch_class_dp2(int la, int lb, int lc, const ClassArgs& a, cudaStream_t s);    // eri_class_dp2.cu
+bool launch_class_dd(int la, int lb, int lc, const ClassArgs& a, cudaStream_t s);     // eri_class_dd.cu
+bool launch_class_fs(int la, int lb, int lc, const ClassArgs& a, cudaStream_t s);     // eri_class_fs.cu
 
 }  // namespace eri
 }  // namespace rr

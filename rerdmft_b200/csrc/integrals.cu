@@ -17,10 +17,10 @@
 // with f(0) = 1/sqrt(4 pi), f(1) = sqrt(3/(4 pi)) and f(l >= 2) = 1.
 //
 // GPU mapping.  Work items are (orbital shell pair, aux shell), grouped by angular-momentum class
-// (l_A >= l_B after swapping the pair).  The low classes, where most primitive triples are (s and p pairs
-// with long contractions), run one thread per item (or per item and aux component) in kernels templated
-// on (l_A, l_B, l_C): E, R and the accumulators in registers, every component and Hermite loop unrolled.
-// The other classes and the metric run one warp per item: per primitive pair lanes 0-2 build the three E
+// (l_A >= l_B after swapping the pair).  The classes up to (dd|f) and (fs|f) run one thread per item (or per
+// item and aux component) in kernels templated on (l_A, l_B, l_C): E, R and the accumulators in registers,
+// every component and Hermite loop unrolled; so does the metric up to (f|f).
+// The other classes run one warp per item: per primitive pair lanes 0-2 build the three E
 // tables in shared memory; per aux primitive lane 3 evaluates the Boys function and the warp builds the R
 // table level by level (in place, one __syncwarp per level); each lane then accumulates its share of the
 // (component a, component b, component c) outputs, in chunks of 32 x kOutPerLane.  The Boys function
@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -329,7 +330,8 @@ __global__ void boys_kernel(const double* T, int64_t count, int nmax, const doub
 
 bool launch_class_any(int la, int lb, int lc, const ClassArgs& a, cudaStream_t s) {
   return launch_class_sp(la, lb, lc, a, s) || launch_class_split(la, lb, lc, a, s) ||
-         launch_class_dp01(la, lb, lc, a, s) || launch_class_dp2(la, lb, lc, a, s);
+         launch_class_dp01(la, lb, lc, a, s) || launch_class_dp2(la, lb, lc, a, s) ||
+         launch_class_dd(la, lb, lc, a, s) || launch_class_fs(la, lb, lc, a, s);
 }
 
 double common_factor(int l) {
@@ -524,26 +526,87 @@ void launch_eri(const DevShells& d, const int2* pairs, int64_t npairs, const int
   RR_LAUNCH_CHECK();
 }
 
-struct IntCtx {
-  cudaStream_t s = nullptr;
-  bool own = false;
-  explicit IntCtx(const rr_opts* o) {
-    if (o && o->stream) {
-      s = static_cast<cudaStream_t>(o->stream);
-    } else {
-      RR_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-      own = true;
+// Streams of one call.  The classes write disjoint outputs, and each kernel alone leaves SMs idle for its last
+// quarter (its longest contractions run 80 primitive pairs in one thread) and most warp slots empty (register-bound
+// occupancy), so they are dealt out to kLanes streams: (H2O)_8 / cc-pVDZ 3.45 -> 2.75 ms of kernels.  A set of
+// streams costs 0.6 ms to make and destroy: sets are handed back for the next call on the device, at most kKept
+// of them wait, and a set is with one call at a time (every call ends with its work done).
+constexpr int kLanes = 4;
+struct StreamSet {
+  int dev = 0;
+  cudaStream_t s[kLanes] = {};
+  cudaEvent_t fork = nullptr, join[kLanes] = {};
+  StreamSet() {
+    dev = current_device();
+    for (auto& x : s) RR_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
+    RR_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    for (auto& e : join) RR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  }
+  ~StreamSet() {
+    for (auto& x : s)
+      if (x) cudaStreamDestroy(x);
+    if (fork) cudaEventDestroy(fork);
+    for (auto& e : join)
+      if (e) cudaEventDestroy(e);
+  }
+};
+struct StreamSets {
+  static constexpr size_t kKept = 8;
+  std::mutex mu;
+  std::vector<std::unique_ptr<StreamSet>> kept;
+  std::unique_ptr<StreamSet> take() {
+    const int dev = current_device();
+    {
+      std::lock_guard<std::mutex> lock(mu);
+      for (auto& k : kept)
+        if (k->dev == dev) {
+          std::swap(k, kept.back());
+          std::unique_ptr<StreamSet> out = std::move(kept.back());
+          kept.pop_back();
+          return out;
+        }
     }
+    return std::unique_ptr<StreamSet>(new StreamSet());
+  }
+  void give(std::unique_ptr<StreamSet> x) {
+    std::lock_guard<std::mutex> lock(mu);
+    if (kept.size() < kKept) kept.push_back(std::move(x));
+  }
+  static StreamSets& get() {
+    static StreamSets* p = new StreamSets();  // never destroyed: streams do not outlive the driver
+    return *p;
+  }
+};
+
+struct IntCtx {
+  std::unique_ptr<StreamSet> set;
+  cudaStream_t s = nullptr;  // the caller's stream, or the set's first
+  int lane = 0;
+  explicit IntCtx(const rr_opts* o) : set(StreamSets::get().take()) {
+    s = o && o->stream ? static_cast<cudaStream_t>(o->stream) : set->s[0];
   }
   ~IntCtx() {
-    if (own && s) {
-      cudaStreamSynchronize(s);
-      cudaStreamDestroy(s);
+    bool done = true;  // after an error too, nothing of this call is left on the streams
+    for (auto x : set->s) done = cudaStreamSynchronize(x) == cudaSuccess && done;
+    if (done) StreamSets::get().give(std::move(set));
+  }
+  cudaStream_t lane_stream(int i) const { return i == 0 ? s : set->s[i]; }
+  // Between fork and join, next() deals out streams ordered after what s holds; after join, s waits for all of them.
+  void fork() {
+    RR_CUDA(cudaEventRecord(set->fork, s));
+    for (int i = 1; i < kLanes; ++i) RR_CUDA(cudaStreamWaitEvent(set->s[i], set->fork, 0));
+  }
+  cudaStream_t next() { return lane_stream(lane++ % kLanes); }
+  void join() {
+    for (int i = 1; i < kLanes; ++i) {
+      RR_CUDA(cudaEventRecord(set->join[i], set->s[i]));
+      RR_CUDA(cudaStreamWaitEvent(s, set->join[i], 0));
     }
   }
 };
 
-void aux_metric_device(const rr_basis* aux, double* M, cudaStream_t s) {
+void aux_metric_device(const rr_basis* aux, double* M, IntCtx& c) {
+  const cudaStream_t s = c.s;
   HostShells hs;
   group_shells(aux, "auxMetric", hs);
   const int na = static_cast<int>(hs.sh.size());
@@ -580,6 +643,7 @@ void aux_metric_device(const rr_basis* aux, double* M, cudaStream_t s) {
   upload(dp, pairs, s);
   upload(dc, cidx, s);
   ClassArgs ca{d.sh.p, d.ex.p, d.co.p, d.fn.p, d.sc.p, nullptr, 0, nullptr, 0, aux->n, M, boys, 1};
+  c.fork();
   for (int la = 0; la <= kMaxL; ++la)
     for (int lc = 0; lc <= kMaxL; ++lc) {
       const int64_t np = p0[la + 1] - p0[la], nc = c0[lc + 1] - c0[lc];
@@ -588,13 +652,16 @@ void aux_metric_device(const rr_basis* aux, double* M, cudaStream_t s) {
       ca.npairs = np;
       ca.cidx = dc.p + c0[lc];
       ca.ncs = nc;
-      if (!launch_class_any(la, 0, lc, ca, s))
-        launch_eri(d, dp.p + p0[la], np, dc.p + c0[lc], nc, hs.lmax, hs.lmax, true, aux->n, M, boys, s);
+      const cudaStream_t ls = c.next();
+      if (!launch_class_any(la, 0, lc, ca, ls))
+        launch_eri(d, dp.p + p0[la], np, dc.p + c0[lc], nc, hs.lmax, hs.lmax, true, aux->n, M, boys, ls);
     }
+  c.join();
   RR_CUDA(cudaStreamSynchronize(s));  // the tables are freed on return
 }
 
-void three_center_raw_device(const rr_basis* orb, const rr_basis* aux, double* raw, cudaStream_t s) {
+void three_center_raw_device(const rr_basis* orb, const rr_basis* aux, double* raw, IntCtx& c) {
+  const cudaStream_t s = c.s;
   HostShells ho, ha;
   group_shells(orb, "threeCenterIntegralsRaw (orbital basis)", ho);
   group_shells(aux, "threeCenterIntegralsRaw (aux basis)", ha);
@@ -639,6 +706,7 @@ void three_center_raw_device(const rr_basis* orb, const rr_basis* aux, double* r
   upload(dp, pairs, s);
   upload(dc, cidx, s);
   ClassArgs ca{d.sh.p, d.ex.p, d.co.p, d.fn.p, d.sc.p, nullptr, 0, nullptr, 0, orb->n, raw, boys, 0};
+  c.fork();
   for (const Range& r : ranges)
     for (int lc = 0; lc <= kMaxL; ++lc) {
       const int64_t nc = c0[lc + 1] - c0[lc];
@@ -647,9 +715,11 @@ void three_center_raw_device(const rr_basis* orb, const rr_basis* aux, double* r
       ca.npairs = r.np;
       ca.cidx = dc.p + c0[lc];
       ca.ncs = nc;
-      if (!launch_class_any(r.la, r.lb, lc, ca, s))
-        launch_eri(d, dp.p + r.p0, r.np, dc.p + c0[lc], nc, ho.lmax, ha.lmax, false, orb->n, raw, boys, s);
+      const cudaStream_t ls = c.next();
+      if (!launch_class_any(r.la, r.lb, lc, ca, ls))
+        launch_eri(d, dp.p + r.p0, r.np, dc.p + c0[lc], nc, ho.lmax, ha.lmax, false, orb->n, raw, boys, ls);
     }
+  c.join();
   RR_CUDA(cudaStreamSynchronize(s));  // the tables are freed on return
 }
 
@@ -690,7 +760,7 @@ int rr_int_aux_metric(const rr_basis* aux, double* metric, const rr_opts* opts) 
       buf.alloc(static_cast<size_t>(n * n));
       M = buf.p;
     }
-    rr::aux_metric_device(aux, M, c.s);
+    rr::aux_metric_device(aux, M, c);
     if (host) {
       RR_CUDA(cudaMemcpyAsync(metric, M, sizeof(double) * n * n, cudaMemcpyDeviceToHost, c.s));
       RR_CUDA(cudaStreamSynchronize(c.s));
@@ -712,7 +782,7 @@ int rr_int_three_center_raw(const rr_basis* basis, const rr_basis* aux, double* 
       buf.alloc(static_cast<size_t>(na * n * n));
       out = buf.p;
     }
-    rr::three_center_raw_device(basis, aux, out, c.s);
+    rr::three_center_raw_device(basis, aux, out, c);
     if (host) {
       RR_CUDA(cudaMemcpyAsync(raw, out, sizeof(double) * na * n * n, cudaMemcpyDeviceToHost, c.s));
       RR_CUDA(cudaStreamSynchronize(c.s));
@@ -730,7 +800,7 @@ int rr_ri_create_basis(const rr_basis* basis, const rr_basis* aux, double metric
     rr::IntCtx c(nullptr);
     rr::DevBuf<double> M(static_cast<size_t>(na * na)), X(static_cast<size_t>(na * na)),
         raw(static_cast<size_t>(na * n * n)), td;
-    rr::aux_metric_device(aux, M.p, c.s);
+    rr::aux_metric_device(aux, M.p, c);
     rr_opts dev{};
     dev.mem = RR_MEM_DEVICE;
     dev.precision = RR_PREC_FP64;
@@ -739,7 +809,7 @@ int rr_ri_create_basis(const rr_basis* basis, const rr_basis* aux, double metric
     int64_t kept = 0;
     rr_rank_report rep{};
     rr::canonical_orthogonalize(M.p, na, false, metric_threshold, X.p, &kept, &rep, &dev);
-    rr::three_center_raw_device(basis, aux, raw.p, c.s);
+    rr::three_center_raw_device(basis, aux, raw.p, c);
     if (t) {
       RR_REQUIRE(n_out >= 1, RR_ERR_ARG, "rr_ri_create_basis: n_out must be >= 1 with t");
       td.alloc(static_cast<size_t>(n * n_out));
