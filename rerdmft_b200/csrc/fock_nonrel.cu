@@ -448,16 +448,23 @@ void fock_nonrel(rr_ri_store* h, const double* hc, const double* D, const double
     const char* e = std::getenv("RR_J_AFTER_RECOVERY");
     return e && std::atoi(e) == 1;
   }();
-  if (host) {
-    auto& c = h->ctx;
-    coulomb_early(h, Dp, J, c.side, j_ctas);
-    copy_in(hd, hc, n2, true, c.side);  // read only by the final combine
-    RR_CUDA(cudaEventRecord(c.upl[2], c.side));
-    h_ready = c.upl[2];
-  } else if (!j_late) {
-    coulomb_early(h, Dp, J, s, j_ctas);
+  cudaEvent_t j_from = nullptr;
+  if (!host && !j_late) {  // the J passes wait for what s holds now, not for the recovery that may be queued before them
+    RR_CUDA(cudaEventRecord(h->ctx.upl[0], s));
+    j_from = h->ctx.upl[0];
   }
-  const int64_t nocc = occupied_ct(h, Xd, Sd, Dp, n, n_eff, 0.5, false, false, Ct, s, d_ready);
+  const int64_t nocc = occupied_ct(h, Xd, Sd, Dp, n, n_eff, 0.5, false, false, Ct, s, d_ready, [&] {
+    auto& c = h->ctx;
+    if (host) {
+      coulomb_early(h, Dp, J, c.side, j_ctas);
+      copy_in(hd, hc, n2, true, c.side);  // read only by the final combine
+      RR_CUDA(cudaEventRecord(c.upl[2], c.side));
+      h_ready = c.upl[2];
+    } else if (j_from) {
+      RR_CUDA(cudaStreamWaitEvent(c.side, j_from, 0));
+      coulomb_early(h, Dp, J, c.side, j_ctas);
+    }
+  });
   if (!host && j_late) coulomb_early(h, Dp, J, s, j_ctas);
   if (d_ready) RR_CUDA(cudaStreamWaitEvent(s, d_ready, 0));  // (n_eff = 0 skips the products)
   prof_mark(h, 1, s);

@@ -202,9 +202,20 @@ void projector_ct(rr_ri_store* h, const double* A, const double* Pe, const doubl
 // Dp: density (n x n, ld n); S (n x n); X (n x n_eff).  d_ready (optional): event s waits on
 // before the first product that reads Dp.  Returns r.
 int64_t occupied_ct(rr_ri_store* h, const double* X, const double* S, const double* Dp, int64_t n, int64_t n_eff,
-                    double scale, bool cplx, bool weighted, double* Ct, cudaStream_t s, cudaEvent_t d_ready) {
+                    double scale, bool cplx, bool weighted, double* Ct, cudaStream_t s, cudaEvent_t d_ready,
+                    const std::function<void()>& between) {
   const int PL = cplx ? 2 : 1;
+  const bool small = n_eff > 0 && recover_small_fits(n, n_eff, cplx);
+  if (between && !small) between();
   if (n_eff == 0) return 0;
+  if (small) {
+    // the small builds wait for the host's launches: this one first, it is the longest part
+    if (d_ready) RR_CUDA(cudaStreamWaitEvent(s, d_ready, 0));
+    recover_small_launch(h, X, S, Dp, n, n_eff, scale, cplx, weighted, Ct, s);
+    if (between) between();
+    int64_t r = 0;
+    if (recover_small_finish(h, s, &r)) return r;
+  }
   double *SD, *Y, *Pe, *A, *T, *A2, *F, *res;
   int* rank;
   Arena ar(&h->solver_a);

@@ -1,6 +1,8 @@
 // The resident RI store behind an rr_ri_handle, and the helpers every entry point shares.
 #pragma once
 
+#include <functional>
+
 #include "gemm_f64.cuh"
 #include "j_stream.cuh"
 #include "mixed.cuh"
@@ -112,9 +114,18 @@ struct RelBuild {
 
 cudaStream_t call_stream(rr_ri_store* h, const rr_opts* o);
 // Occupied-orbital recovery (recovery.cu): c_t (r x n) from the density; returns r.  d_ready
-// (optional): event s waits on before the first product that reads Dp.
+// (optional): event s waits on before the first product that reads Dp.  between (optional): called once, after the
+// recovery's work is queued where that is one launch, else before it; queues work that may run beside it on other streams.
 int64_t occupied_ct(rr_ri_store* h, const double* X, const double* S, const double* Dp, int64_t n, int64_t n_eff,
-                    double scale, bool cplx, bool weighted, double* Ct, cudaStream_t s, cudaEvent_t d_ready = nullptr);
+                    double scale, bool cplx, bool weighted, double* Ct, cudaStream_t s, cudaEvent_t d_ready = nullptr,
+                    const std::function<void()>& between = nullptr);
+// occupied_ct in one launch on one CTA (recover_small.cu), for matrices that fit its shared memory four at a time; nothing
+// between the two calls may use solver_a.  finish waits for s and returns false when r turned out too large a part of
+// n_eff (Ct not written).
+bool recover_small_fits(int64_t n, int64_t n_eff, bool cplx);
+void recover_small_launch(rr_ri_store* h, const double* X, const double* S, const double* D, int64_t n, int64_t n_eff, double scale,
+                          bool cplx, bool weighted, double* ct, cudaStream_t s);
+bool recover_small_finish(rr_ri_store* h, cudaStream_t s, int64_t* r);
 // Builds h->Bpk[t] from h->B[t] (n x n rows) when it fits; synchronises s.
 void pack_for_j(rr_ri_store* h, int t, int64_t n, cudaStream_t s);
 // JTensor of tensor t (n x n rows) over the packed copy when there is one (D folded into dfold at
