@@ -226,27 +226,49 @@ __global__ void __maxnreg__(48) j_pass2_kernel(const P2 p) {
 
 __host__ __device__ inline int64_t out_len(const JTensor& t) { return t.tri_n ? t.tri_n * t.tri_n : t.len; }
 
-// J[t][k] from the pass-2 partials of entry k (packed rows: of entry tri_index(min, max), so both
-// triangles get the same sum, added in the same order).
-__global__ void j_finish_kernel(JTensor t0, JTensor t1, int ntens, int nrange, int64_t jstride, const double* jpart,
-                                double scale) {
-  const int64_t out0 = out_len(t0);
-  const int64_t total = out0 + (ntens > 1 ? out_len(t1) : 0);
-  for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < total;
-       k += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const bool second = k >= out0;
-    const JTensor& t = second ? t1 : t0;
-    const int64_t kk = second ? k - out0 : k;
-    int64_t src = second ? t0.len : 0;
-    if (t.tri_n) {
-      const int64_t q = kk / t.tri_n, a = kk - q * t.tri_n;
-      src += q <= a ? tri_index(q, a, t.tri_n) : tri_index(a, q, t.tri_n);
-    } else {
-      src += kk;
-    }
+// J[t] from the pass-2 partials.  A CTA sums 32 consecutive entries of the partials, warp w the ranges w, w + 8, ...
+// (the eight sums are added in the order of the warps); a packed entry (q, a) goes to both triangles.  Bound:
+// reading the partials once, nrange of them an entry (n = 160: 36 - 592 ranges of 103 KB).  With a thread per output
+// element instead, the lower triangle read the packed rows column-wise and each thread walked all the ranges:
+// n = 160 beside the exchange products 169 us, now below 20; n = 400 65 us, now 19; X2C nl = 200 205 us, now 46.
+constexpr int kFinishWarps = 8;
+__global__ void __launch_bounds__(32 * kFinishWarps) j_finish_kernel(JTensor t0, JTensor t1, int ntens, int nrange, int64_t jstride,
+                                                                     const double* jpart, double scale) {
+  __shared__ double part[kFinishWarps][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int64_t k0 = blockIdx.x * 32LL; k0 < jstride; k0 += gridDim.x * 32LL) {
+    const int64_t k = k0 + lane;
     double s = 0.0;
-    for (int r = 0; r < nrange; ++r) s += jpart[r * jstride + src];
-    t.J[kk] = scale * s;
+    if (k < jstride) {
+#pragma unroll 8
+      for (int r = w; r < nrange; r += kFinishWarps) s += jpart[r * jstride + k];
+    }
+    part[w][lane] = s;
+    __syncthreads();
+    if (w == 0 && k < jstride) {
+      s = part[0][lane];
+#pragma unroll
+      for (int i = 1; i < kFinishWarps; ++i) s += part[i][lane];
+      s *= scale;
+      const bool second = k >= t0.len;
+      const JTensor& t = second ? t1 : t0;
+      const int64_t kk = second ? k - t0.len : k;
+      if (t.tri_n) {
+        // row q of the triangle starts at q (2 n - q + 1) / 2: the root of that, then the exact row beside it
+        const int64_t n = t.tri_n;
+        const double h = n + 0.5;
+        int64_t q = static_cast<int64_t>(h - sqrt(fmax(0.0, h * h - 2.0 * static_cast<double>(kk))));
+        q = max(static_cast<int64_t>(0), min(q, n - 1));
+        while (q > 0 && tri_index(q, q, n) > kk) --q;
+        while (q + 1 < n && tri_index(q + 1, q + 1, n) <= kk) ++q;
+        const int64_t a = q + (kk - tri_index(q, q, n));
+        t.J[q * n + a] = s;
+        t.J[a * n + q] = s;
+      } else {
+        t.J[kk] = s;
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -399,18 +421,17 @@ void j_pass2(const JPlan& pl, const double* gpart, double* jpart, int* err, cuda
 
 void j_finish(const JPlan& pl, const double* jpart, double scale, cudaStream_t s) {
   const int64_t jstride = pl.t[0].len + (pl.ntens > 1 ? pl.t[1].len : 0);
-  const int64_t total = out_len(pl.t[0]) + (pl.ntens > 1 ? out_len(pl.t[1]) : 0);
-  if (total == 0) return;
+  if (jstride == 0) return;
   // nrange actually used by pass 2 (ranges past naux produce no rows and are never read).
   const int64_t rp = (pl.naux + pl.nrange - 1) / std::max(pl.nrange, 1);
   const int used = pl.naux ? static_cast<int>((pl.naux + rp - 1) / rp) : 0;
-  const int blocks = static_cast<int>(std::min<int64_t>(4LL * sm_count(), (total + 255) / 256));
+  const int blocks = static_cast<int>(std::min<int64_t>(8LL * sm_count(), (jstride + 31) / 32));
   if (used == 0) {
     RR_CUDA(cudaMemsetAsync(pl.t[0].J, 0, sizeof(double) * out_len(pl.t[0]), s));
     if (pl.ntens > 1) RR_CUDA(cudaMemsetAsync(pl.t[1].J, 0, sizeof(double) * out_len(pl.t[1]), s));
     return;
   }
-  j_finish_kernel<<<blocks, 256, 0, s>>>(pl.t[0], pl.t[1], pl.ntens, used, jstride, jpart, scale);
+  j_finish_kernel<<<blocks, 32 * kFinishWarps, 0, s>>>(pl.t[0], pl.t[1], pl.ntens, used, jstride, jpart, scale);
   RR_LAUNCH_CHECK();
 }
 
