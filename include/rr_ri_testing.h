@@ -78,6 +78,14 @@ int rr_test_drop_digit_planes(void* ri_handle, int32_t* had);
 int rr_test_chol_apply(const double* M, int64_t r, const double* Y, int64_t n, int32_t cplx, int32_t times_l, double* out,
                        int32_t* ran, int32_t* status);
 
+/* The one-launch SP2 purification: X <- the projector onto the lowest nocc eigenvectors of the Hermitian F (n x n, interleaved
+ * when cplx) from the spectral interval [lo, hi]; sure: the interval holds the spectrum.  *outcome: 0 converged, 1 the interval
+ * missed part of the spectrum or max_steps passed, 2 a grid barrier expired. */
+int rr_test_sp2(const double* F, int64_t n, double nocc, int32_t cplx, double lo, double hi, int32_t sure, int32_t max_steps,
+                double* X, double* outcome);
+/* [lo, hi] (host, in and out) narrowed to the widened extreme eigenvalues of T y = theta M y (32 x 32). */
+int rr_test_ritz(const double* T, const double* M, int32_t cplx, double* lo_hi);
+
 /* Failure detection without a fault: one CTA of `threads` threads waits on an mbarrier that nothing
  * arrives on (and no bulk copy is in flight) through the bounded wait every TMA pipeline of the library
  * uses, with `spin_limit` polls (1 .. 4,194,304, the pipelines' own limit).  The wait expires, records

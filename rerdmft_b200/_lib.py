@@ -173,6 +173,8 @@ _SIGS = {
     "rr_ri_create_basis": (ctypes.c_int, [ctypes.POINTER(Basis), ctypes.POINTER(Basis), _d, _vp, _i64,
                                           ctypes.POINTER(_vp), ctypes.POINTER(_i64), ctypes.POINTER(RankReport)]),
     "rr_test_chol_apply": (ctypes.c_int, [_vp, _i64, _vp, _i64, _i32, _i32, _vp, _vp, _vp]),
+    "rr_test_sp2": (ctypes.c_int, [_vp, _i64, _d, _i32, _d, _d, _i32, _i32, _vp, _vp]),
+    "rr_test_ritz": (ctypes.c_int, [_vp, _vp, _i32, _vp]),
     "rr_test_boys": (ctypes.c_int, [_vp, _i64, _i32, _vp]),
     "rr_ri_info": (ctypes.c_int, [_vp, ctypes.POINTER(_i64), ctypes.POINTER(_i64), ctypes.POINTER(_i64)]),
     "rr_ri_sync": (ctypes.c_int, [_vp]),

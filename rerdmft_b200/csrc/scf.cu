@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "ri_store.cuh"
+#include "sp2.cuh"
 
 namespace rr {
 
@@ -476,17 +477,6 @@ __global__ void normalize_cols_kernel(double* K, int64_t n, int ldk, int c0) {
     for (int q = 0; q < PL; ++q) K[(r * ldk + c) * PL + q] *= scale;
 }
 
-// b = [lo, hi] (the Gershgorin interval on entry) narrowed to the Ritz interval widened by 10% of
-// its spread on both sides, when the small eigenproblem succeeded.
-__global__ void ritz_bounds_kernel(const double* w, int k, const int* info, double* b) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const double lo = w[0], hi = w[k - 1], spread = hi - lo;
-  if (*info != 0 || !(spread >= 0.0) || !isfinite(lo) || !isfinite(hi)) return;
-  const double m = 0.1 * spread + 1e-12 * fmax(fabs(lo), fabs(hi));
-  const double nlo = fmax(b[0], lo - m), nhi = fmin(b[1], hi + m);
-  if (nhi > nlo) { b[0] = nlo; b[1] = nhi; }
-}
-
 }  // namespace
 
 bool diis_solve(const std::vector<double>& m, const std::vector<double>& rhs, size_t n, double tol,
@@ -497,18 +487,18 @@ bool diis_solve(const std::vector<double>& m, const std::vector<double>& rhs, si
 // Narrows the SP2 spectral interval b (device, [lo, hi], Gershgorin on entry) of the Hermitian n x n
 // F with the Ritz values of F on the block Krylov space [V, F V, F^2 V, F^3 V] (V: 8 fixed
 // pseudo-random vectors), widened by 10% of their spread: a generalized 32 x 32 eigenproblem
-// (K^dagger F K) y = theta (K^dagger K) y on the device (cuSOLVER).  Small matrices keep b.
+// (K^dagger F K) y = theta (K^dagger K) y on the device (sp2.cu).  Small matrices keep b.
 void ritz_bounds(rr_ri_store* h, const double* F, int64_t n, bool cplx, double* b, cudaStream_t s) {
   constexpr int m = 8, q = 4, k = m * q;
+  static_assert(k == kRitz, "size of the small eigenproblem");
   if (n < 4 * k) return;
   const int PL = cplx ? 2 : 1;
-  double *K, *FK, *T, *M, *w;
+  double *K, *FK, *T, *M;
   Arena ar(&h->solver_a);
   ar.request(&K, n * k * PL);
   ar.request(&FK, n * k * PL);
   ar.request(&T, k * k * PL);
   ar.request(&M, k * k * PL);
-  ar.request(&w, k);
   ar.commit();
   if (cplx) krylov_start_kernel<2><<<blocks_for(n * m * 2), 256, 0, s>>>(K, n, k, m);
   else krylov_start_kernel<1><<<blocks_for(n * m), 256, 0, s>>>(K, n, k, m);
@@ -536,28 +526,7 @@ void ritz_bounds(rr_ri_store* h, const double* F, int64_t n, bool cplx, double* 
   t.B = K; t.C = M;
   t.mirror = 1;
   gemm(t, s, h->work.p, static_cast<int64_t>(h->work.n));
-  auto& c = h->ctx;
-  RR_SOLVER(cusolverDnSetStream(c.solver_handle(), s));
-  c.solver_info.ensure(1);
-  int lwork = 0;
-  if (cplx) {
-    auto* tz = reinterpret_cast<cuDoubleComplex*>(T);
-    auto* mz = reinterpret_cast<cuDoubleComplex*>(M);
-    RR_SOLVER(cusolverDnZhegvd_bufferSize(c.solver, CUSOLVER_EIG_TYPE_1, CUSOLVER_EIG_MODE_NOVECTOR,
-                                          CUBLAS_FILL_MODE_UPPER, k, tz, k, mz, k, w, &lwork));
-    c.solver_work.ensure(2 * static_cast<size_t>(lwork) + 2);
-    RR_SOLVER(cusolverDnZhegvd(c.solver, CUSOLVER_EIG_TYPE_1, CUSOLVER_EIG_MODE_NOVECTOR, CUBLAS_FILL_MODE_UPPER, k,
-                               tz, k, mz, k, w, reinterpret_cast<cuDoubleComplex*>(c.solver_work.p), lwork,
-                               c.solver_info.p));
-  } else {
-    RR_SOLVER(cusolverDnDsygvd_bufferSize(c.solver, CUSOLVER_EIG_TYPE_1, CUSOLVER_EIG_MODE_NOVECTOR,
-                                          CUBLAS_FILL_MODE_UPPER, k, T, k, M, k, w, &lwork));
-    c.solver_work.ensure(static_cast<size_t>(lwork) + 1);
-    RR_SOLVER(cusolverDnDsygvd(c.solver, CUSOLVER_EIG_TYPE_1, CUSOLVER_EIG_MODE_NOVECTOR, CUBLAS_FILL_MODE_UPPER, k, T,
-                               k, M, k, w, c.solver_work.p, lwork, c.solver_info.p));
-  }
-  ritz_bounds_kernel<<<1, 32, 0, s>>>(w, k, c.solver_info.p, b);
-  RR_LAUNCH_CHECK();
+  ritz_interval(T, M, cplx, b, s);
 }
 
 // SP2 purification: projector (n x n, into Pi) onto the lowest `nocc` eigenvectors of the symmetric
@@ -579,6 +548,21 @@ void sp2_projector(rr_ri_store* h, const double* F, int64_t n, int64_t nocc, dou
   // Gershgorin interval kept in scal[4..5]; the Ritz interval (tighter: fewer SP2 steps) is tried first
   RR_CUDA(cudaMemcpyAsync(scal + 4, scal, 2 * sizeof(double), cudaMemcpyDeviceToDevice, s));
   ritz_bounds(h, F, n, cplx, scal, s);
+  const double N = static_cast<double>(nocc);
+  if (n <= (cplx ? kSp2MaxComplex : kSp2MaxReal)) {
+    // all steps in one launch (sp2.cu): from the Ritz interval, and from Gershgorin's if that missed part of the spectrum
+    double outcome = 1.0;
+    for (int sure = 0; sure < 2 && outcome == 1.0; ++sure) {
+      if (sure) RR_CUDA(cudaMemcpyAsync(scal, scal + 4, 2 * sizeof(double), cudaMemcpyDeviceToDevice, s));
+      double* got = part + sp2_scratch_doubles();
+      sp2_run(F, n, N, cplx, scal, sure != 0, sure ? 120 : 60, Pi, T, part, got, s);
+      RR_CUDA(cudaMemcpyAsync(&outcome, got, sizeof(double), cudaMemcpyDeviceToHost, s));
+      host_wait(h, s);
+    }
+    RR_REQUIRE(outcome != 2.0, RR_ERR_TIMEOUT, "SCF: a grid barrier of the density purification expired");
+    RR_REQUIRE(outcome == 0.0, RR_ERR_SOLVER, "SCF: density purification did not converge (no gap at the Fermi level?)");
+    return;
+  }
   // ping-pong partials of X after the Gershgorin partials (the GEMM's split-K scratch follows them)
   double* sp_part[2] = {part + 2 * RED_CTAS, part + 4 * RED_CTAS};
   auto init = [&] {
@@ -592,7 +576,6 @@ void sp2_projector(rr_ri_store* h, const double* F, int64_t n, int64_t nocc, dou
   g.M = n; g.N = n; g.K = n;
   g.A = Pi; g.lda = n; g.B = Pi; g.ldb = n; g.C = T; g.ldc = n;
   g.mirror = 1;  // X is Hermitian, so is X^2: upper tiles, the rest mirrored
-  const double N = static_cast<double>(nocc);
   double* gw = part + 6 * RED_CTAS;  // split-K scratch of the X^2 products
   const int64_t gcap = static_cast<int64_t>(h->work.n) - 6 * RED_CTAS;
   bool gershgorin = false;

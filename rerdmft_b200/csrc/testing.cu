@@ -4,6 +4,7 @@
 
 #include "chol.cuh"
 #include "ri_store.cuh"
+#include "sp2.cuh"
 #include "gemm_f64.cuh"
 #include "tma_util.cuh"
 
@@ -98,6 +99,38 @@ int rr_test_chol_apply(const double* M, int64_t r, const double* Y, int64_t n, i
     RR_CUDA(cudaMemset(st.p, 0, sizeof(int)));
     *ran = rr::chol_apply(M, r, Y, n, cplx != 0, times_l != 0, out, st.p, nullptr) ? 1 : 0;
     RR_CUDA(cudaMemcpy(status, st.p, sizeof(int), cudaMemcpyDeviceToHost));
+    return RR_OK;
+  } catch (const rr::Error& e) {
+    rr::set_last_error(e.what());
+    return e.code;
+  }
+}
+
+int rr_test_sp2(const double* F, int64_t n, double nocc, int32_t cplx, double lo, double hi, int32_t sure, int32_t max_steps,
+                double* X, double* outcome) {
+  try {
+    rr::set_last_error("");
+    RR_REQUIRE(F && X && outcome && n >= 1 && n <= (cplx ? rr::kSp2MaxComplex : rr::kSp2MaxReal), RR_ERR_ARG, "rr_test_sp2: bad argument");
+    const double b[2] = {lo, hi};
+    rr::DevBuf<double> db(2), Y(static_cast<size_t>(n * n * (cplx ? 2 : 1))), w(static_cast<size_t>(rr::sp2_scratch_doubles()) + 4);
+    RR_CUDA(cudaMemcpy(db.p, b, sizeof(b), cudaMemcpyHostToDevice));
+    rr::sp2_run(F, n, nocc, cplx != 0, db.p, sure != 0, max_steps, X, Y.p, w.p, w.p + rr::sp2_scratch_doubles(), nullptr);
+    RR_CUDA(cudaMemcpy(outcome, w.p + rr::sp2_scratch_doubles(), sizeof(double), cudaMemcpyDeviceToHost));
+    return RR_OK;
+  } catch (const rr::Error& e) {
+    rr::set_last_error(e.what());
+    return e.code;
+  }
+}
+
+int rr_test_ritz(const double* T, const double* M, int32_t cplx, double* lo_hi) {
+  try {
+    rr::set_last_error("");
+    RR_REQUIRE(T && M && lo_hi, RR_ERR_ARG, "rr_test_ritz: null argument");
+    rr::DevBuf<double> db(2);
+    RR_CUDA(cudaMemcpy(db.p, lo_hi, 2 * sizeof(double), cudaMemcpyHostToDevice));
+    rr::ritz_interval(T, M, cplx != 0, db.p, nullptr);
+    RR_CUDA(cudaMemcpy(lo_hi, db.p, 2 * sizeof(double), cudaMemcpyDeviceToHost));
     return RR_OK;
   } catch (const rr::Error& e) {
     rr::set_last_error(e.what());
