@@ -105,8 +105,16 @@ bool batched_tile80(int64_t M, int64_t N, int64_t batch) {
 // split-K: more CTAs and no reduction launch; measured 14 us instead of 20 us at n = 400.
 bool use_tile32(int64_t M, int64_t N, int64_t K) { return M > 48 && M <= 512 && N <= 512 && K <= 2048; }
 
+// Single small products of at most 48 rows (the Gram matrices and coefficient rows of the recovery, the exchange of
+// small systems): 32 x 32 tiles with K split into ranges of 64, where the row-wide tiles below left one to three CTAs
+// walking all of K: r = 37, n = 203: 22 us a product, now 5 + 3 with the reduction.
+bool skinny_tile32(int64_t M, int64_t N, int64_t K, int64_t batch) {
+  return M <= 48 && N <= 512 && K <= 2048 && batch == 1;
+}
+
 template <bool AK, bool BKM>
 void launch_real(const Params& p, dim3 grid, cudaStream_t s) {
+  if (skinny_tile32(p.M, p.N, p.K, p.batch)) return launch_cfg<2, 2, 2, 2, AK, BKM, false>(p, grid, s);
   if (batched_tile80(p.M, p.N, p.batch)) return launch_cfg<5, 5, 2, 2, AK, BKM, false>(p, grid, s);
   if (use_tile32(p.M, p.N, p.K)) return launch_cfg<2, 2, 2, 2, AK, BKM, false>(p, grid, s);
   if (p.M <= 48) {
@@ -130,6 +138,7 @@ bool cplx_tile32(const GemmDesc& d) { return d.cplx && d.M <= 1024 && d.N <= 102
 Shape pick_shape(const GemmDesc& d) {
   if (cplx_tile32(d)) return {32, 32};
   if (d.cplx) return {32, 64};
+  if (skinny_tile32(d.M, d.N, d.K, d.batch)) return {32, 32};
   if (batched_tile80(d.M, d.N, d.batch)) return {80, 80};
   if (use_tile32(d.M, d.N, d.K)) return {32, 32};
   // 33..40 rows (the half-transform at 40 occupied orbitals): 40 x 80 tiles of five 40 x 16 warps,
@@ -148,8 +157,10 @@ int pick_splits(const GemmDesc& d, Shape sh, int64_t* kchunk) {
   const int64_t target = (d.mirror ? 8LL : 16LL) * num_sms();
   int splits = 1;
   if (cplx_tile32(d) || (sh.bm == 32 && sh.bn == 32 && tiles < 2LL * num_sms())) {
-    // small square products (recovery, SCF): one wave of 32 x 32 tiles at most, so split K up to 4
-    splits = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(4, d.K / (4 * KT))));
+    // small products (recovery, SCF): one wave of 32 x 32 tiles at most, so split K up to 4; up to 8, 16 where that
+    // still leaves SMs idle
+    const int64_t most = 16 * tiles <= num_sms() ? 16 : 8 * tiles <= num_sms() ? 8 : 4;
+    splits = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(most, d.K / (4 * KT))));
   } else if (!(sh.bm == 32 && sh.bn == 32) && tiles < 2LL * num_sms() && d.K >= 8 * KT) {
     splits = static_cast<int>(std::min<int64_t>((target + tiles - 1) / tiles, d.K / (8 * KT)));
     splits = std::max(1, std::min(splits, 128));
