@@ -23,6 +23,7 @@
 
 #include "chol.cuh"
 #include "grouped.cuh"
+#include "sp2.cuh"
 #include "ri_store.cuh"
 
 namespace rr {
@@ -494,7 +495,7 @@ struct GroupCtx {
   std::mutex mu;
   cudaStream_t s = nullptr;
   TableRing ring;
-  DevBuf<double> work, scal_all;
+  DevBuf<double> work, scal_all, sp2;
   DevBuf<int> status_all;
   cudaEvent_t ev[4] = {};
 };
@@ -1013,46 +1014,73 @@ void scf_x2c_grouped(rr_x2c_instance* ins, int64_t count, const rr_scf_opts* so,
     GLAUNCH(k_gersh_part, GRC, na, tab, al);
     GLAUNCH(k_reduce<1>, 1, na, tab, al, P_GB, GRC, GRC, 1, 4, 1.0);
     GLAUNCH(k_reduce<2>, 1, na, tab, al, P_GB + GRC, GRC, GRC, 1, 5, 1.0);
-    GLAUNCH(k_sp2_init, GRC, na, tab, al);
     {
       std::vector<int> sp = act;
-      const int* spl = al;
-      // the same X^2 products every step: built once per stretch between read-backs, then re-launched
-      GroupedPlan sq;
-      bool sq_valid = false;
-      for (int step = 0; step < 120 && !sp.empty(); ++step) {
-        sp2_max = std::max<int64_t>(sp2_max, step + 1);
-        if (!sq_valid) {
-          g.clear();
-          for (int i : sp) {
-            const GDev& d = b.gs[i].d;
-            GemmDesc q = cg(d.ne, d.ne, d.ne, d.Pi, d.ne, d.Pi, d.ne, d.T2, d.ne);
-            q.mirror = 2;  // X^2 is Hermitian: upper tiles only, k_sp2_step reads the rest as the mirror
-            g.push_back(q);
-          }
-          const auto t0 = std::chrono::steady_clock::now();
-          gemm_grouped_plan(g, b.s, b.ring, b.work, sq);
-          b.gemm_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-          sq_valid = true;
+      int64_t widest = 0;
+      for (int i : act) widest = std::max(widest, b.gs[i].d.ne);
+      if (widest <= kSp2MaxComplex) {
+        // all steps of all instances in one launch (sp2.cu): 120 steps of a grouped product, a step launch and a host check
+        // every fourth step took 4.7 ms of a scan of 12 instances of 40 - 144 spinors, this 1.4
+        const int64_t per = sp2_scratch_doubles() + 4;
+        b.c.sp2.ensure(static_cast<size_t>(per) * b.gs.size());
+        std::vector<Sp2Problem> q;
+        for (int i : sp) {
+          const GDev& d = b.gs[i].d;
+          double* w = b.c.sp2.p + per * i;
+          q.push_back(Sp2Problem{d.Fo, d.scal + 4, d.Pi, d.T2, w, w + sp2_scratch_doubles(), static_cast<double>(d.r), d.ne});
         }
-        {
-          const auto t0 = std::chrono::steady_clock::now();
-          gemm_grouped_exec(sq, b.s, nullptr);
-          b.gemm_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+        sp2_run_group(q.data(), static_cast<int>(q.size()), [&](const void* t, size_t bytes) { return b.ring.put(t, bytes, b.s); }, b.s);
+        std::vector<double> got(4 * b.gs.size());
+        RR_CUDA(cudaMemcpy2DAsync(got.data(), 4 * sizeof(double), b.c.sp2.p + sp2_scratch_doubles(), per * sizeof(double),
+                                  4 * sizeof(double), b.gs.size(), cudaMemcpyDeviceToHost, b.s));
+        b.sync_scalars();
+        std::vector<int> keep;
+        for (int i : sp) {
+          RR_REQUIRE(got[4 * i] != 2.0, RR_ERR_TIMEOUT, "rr_scf_run_x2c_grouped: a grid barrier of the density purification expired");
+          if (got[4 * i] != 0.0) keep.push_back(i);
+          sp2_max = std::max<int64_t>(sp2_max, static_cast<int64_t>(got[4 * i + 3]));
         }
-        const int pin = (step & 1) ? P_S1 : P_S0, pout = (step & 1) ? P_S0 : P_S1;
-        GLAUNCH(k_sp2_step, GRC, sp.size(), tab, spl, pin, pout);
-        if (step % 4 == 3) {
-          b.sync_scalars();
-          tab = b.upload_tab();
-          std::vector<int> keep;
-          for (int i : sp) {
-            const double t1 = b.gs[i].scal_host[2], t2 = b.gs[i].scal_host[3], N = static_cast<double>(b.gs[i].d.r);
-            if (!(std::fabs(t1 - t2) < 1e-11 * std::max(1.0, N) && std::fabs(t1 - N) < 1e-6)) keep.push_back(i);
+        sp.swap(keep);
+      } else {
+        GLAUNCH(k_sp2_init, GRC, na, tab, al);
+        const int* spl = al;
+        // the same X^2 products every step: built once per stretch between read-backs, then re-launched
+        GroupedPlan sq;
+        bool sq_valid = false;
+        for (int step = 0; step < 120 && !sp.empty(); ++step) {
+          sp2_max = std::max<int64_t>(sp2_max, step + 1);
+          if (!sq_valid) {
+            g.clear();
+            for (int i : sp) {
+              const GDev& d = b.gs[i].d;
+              GemmDesc q = cg(d.ne, d.ne, d.ne, d.Pi, d.ne, d.Pi, d.ne, d.T2, d.ne);
+              q.mirror = 2;  // X^2 is Hermitian: upper tiles only, k_sp2_step reads the rest as the mirror
+              g.push_back(q);
+            }
+            const auto t0 = std::chrono::steady_clock::now();
+            gemm_grouped_plan(g, b.s, b.ring, b.work, sq);
+            b.gemm_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+            sq_valid = true;
           }
-          sp.swap(keep);
-          spl = b.upload_list(sp);
-          sq_valid = false;  // the read-back reset the table space
+          {
+            const auto t0 = std::chrono::steady_clock::now();
+            gemm_grouped_exec(sq, b.s, nullptr);
+            b.gemm_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+          }
+          const int pin = (step & 1) ? P_S1 : P_S0, pout = (step & 1) ? P_S0 : P_S1;
+          GLAUNCH(k_sp2_step, GRC, sp.size(), tab, spl, pin, pout);
+          if (step % 4 == 3) {
+            b.sync_scalars();
+            tab = b.upload_tab();
+            std::vector<int> keep;
+            for (int i : sp) {
+              const double t1 = b.gs[i].scal_host[2], t2 = b.gs[i].scal_host[3], N = static_cast<double>(b.gs[i].d.r);
+              if (!(std::fabs(t1 - t2) < 1e-11 * std::max(1.0, N) && std::fabs(t1 - N) < 1e-6)) keep.push_back(i);
+            }
+            sp.swap(keep);
+            spl = b.upload_list(sp);
+            sq_valid = false;  // the read-back reset the table space
+          }
         }
       }
       for (int i : sp) {  // no gap at the Fermi level

@@ -3,9 +3,9 @@
 // sp2_kernel: all SP2 steps in one cooperative launch.  A step of an n x n matrix is one product X X (16 x 16 tiles of the
 // upper triangle dealt out to the CTAs, FP64 mma.sync m8n8k4: tcgen05 has no FP64 kind) whose epilogue applies the step and writes both triangles,
 // then one grid barrier.  X is Hermitian, so both operands of a tile are rows of X.  The choice between X^2 and
-// 2 X - X^2 needs tr X and tr X^2 = ||X||_F^2 of the matrix being squared, which its writers left as per-CTA
+// 2 X - X^2 needs tr X and tr X^2 = ||X||_F^2 of the matrix being squared, which its writers left as per-tile
 // partials: every CTA adds all of them in the same order and comes to the same choice.
-// Bound: latency (the barrier, one L2 round trip for the rows, a chain of n / 8 mma).  n = 160: 6 us a step
+// Bound: latency (the barrier, one L2 round trip for the rows, a chain of n / 8 mma).  n = 160: 4.4 us a step
 // against 15 us for product, split-K reduction and step kernel, and no host check every fourth step.
 //
 // ritz_kernel: the extreme eigenvalues of a 32 x 32 generalized problem on one CTA: Cholesky reduction
@@ -13,6 +13,7 @@
 // counts (Barth, Martin, Wilkinson, "Calculation of the eigenvalues of a symmetric tridiagonal matrix by the method of bisection",
 // Numer. Math. 9, 1967), 32 points a pass, one warp for either end.  80 us (n = 160, real) against 320 us for the library's sygvd.
 #include <algorithm>
+#include <vector>
 
 #include "chol_rows.cuh"
 #include "sp2.cuh"
@@ -23,14 +24,15 @@ namespace {
 
 constexpr int TILE = 16, SP2_THREADS = 256;
 constexpr int kSp2Smem = 200 * 1024;
-constexpr int kMaxCtas = 256;
+constexpr int kMaxTiles = (kSp2MaxReal / TILE) * (kSp2MaxReal / TILE + 1) / 2;
+constexpr int kMaxGroupCtas = 1184;  // of one launch
 constexpr unsigned kBarrierPolls = 1u << 21;  // about a second
 
 struct Sp2Args {
   const double* F;
   const double* b;
   double *X, *Y;
-  double* part;       // two sets of (tr, fro) per CTA
+  double* part;       // two sets of (tr, fro) per tile
   unsigned* bar;      // zeroed counter, expiry flag
   double* outcome;
   double nocc;
@@ -77,20 +79,36 @@ __device__ __forceinline__ void square_tile(const double* X, int n, int kc, int 
   for (int k0 = 0; k0 < n; k0 += kc) {
     const int kn = min(kc, n - k0), kp = (kn + 7) / 8 * 8;
     __syncthreads();
-    for (int r = w; r < 2 * TILE; r += SP2_THREADS / 32) {
-      const int row = r < TILE ? i0 + r : j0 + r - TILE;
-      double* dst = (r < TILE ? sa : sb) + (r % TILE) * pitch;
-      const double* src = X + (static_cast<int64_t>(row) * n + k0) * PL;
+    // warp w: rows w and w + 8 of either operand, four rows' loads in flight for each of its columns
+    constexpr int NW = SP2_THREADS / 32, NROW = 2 * TILE / NW;
+    const double* src[NROW];
+    double* dst[NROW];
+    bool live[NROW];
+#pragma unroll
+    for (int q = 0; q < NROW; ++q) {
+      const int r = w + NW * q, row = r < TILE ? i0 + r : j0 + r - TILE;
+      live[q] = row < n;
+      dst[q] = (r < TILE ? sa : sb) + (r % TILE) * pitch;
+      src[q] = X + (static_cast<int64_t>(live[q] ? row : 0) * n + k0) * PL;
+    }
 #pragma unroll 4
-      for (int k = lane; k < kp; k += 32) {
-        const bool in = row < n && k < kn;
+    for (int k = lane; k < kp; k += 32) {
+      double v[NROW][PL];
+#pragma unroll
+      for (int q = 0; q < NROW; ++q) {
+        const bool in = live[q] && k < kn;
         if constexpr (PL == 1) {
-          dst[k] = in ? src[k] : 0.0;
+          v[q][0] = in ? src[q][k] : 0.0;
         } else {
-          const double2 v = in ? *reinterpret_cast<const double2*>(src + 2 * k) : make_double2(0.0, 0.0);
-          dst[k] = v.x;
-          dst[TILE * pitch + k] = v.y;
+          const double2 d = in ? *reinterpret_cast<const double2*>(src[q] + 2 * k) : make_double2(0.0, 0.0);
+          v[q][0] = d.x;
+          v[q][PL - 1] = d.y;
         }
+      }
+#pragma unroll
+      for (int q = 0; q < NROW; ++q) {
+        dst[q][k] = v[q][0];
+        if (PL == 2) dst[q][TILE * pitch + k] = v[q][PL - 1];
       }
     }
     __syncthreads();
@@ -140,50 +158,71 @@ __device__ __forceinline__ void square_tile(const double* X, int n, int kc, int 
   __syncthreads();
 }
 
-__device__ __forceinline__ double cta_sum(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+// (a, b) summed over the CTA, in every thread.
+__device__ __forceinline__ void cta_sum2(double& a, double& b, double* red) {
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+  }
   __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  if ((threadIdx.x & 31) == 0) {
+    red[2 * (threadIdx.x >> 5)] = a;
+    red[2 * (threadIdx.x >> 5) + 1] = b;
+  }
   __syncthreads();
-  v = red[0];
-  for (int w = 1; w < SP2_THREADS / 32; ++w) v += red[w];
-  return v;
+  a = red[0];
+  b = red[1];
+  for (int w = 1; w < SP2_THREADS / 32; ++w) {
+    a += red[2 * w];
+    b += red[2 * w + 1];
+  }
+}
+
+// Upper-triangle tile t of nt x nt.
+__device__ __forceinline__ void tile_at(int t, int nt, int& i0, int& j0) {
+  int ti = 0;
+  while (t >= nt - ti) {
+    t -= nt - ti;
+    ++ti;
+  }
+  i0 = ti * TILE;
+  j0 = (ti + t) * TILE;
 }
 
 // X is indexed by element (i n + j) PL; Hermitian to the last bit (both triangles are written from one value).
 template <int PL>
-__global__ void __launch_bounds__(SP2_THREADS, 1) sp2_kernel(const Sp2Args g) {
-  extern __shared__ __align__(16) double sm[];
-  __shared__ double red[TILE * 17 * PL], tile[TILE * 17 * PL], sums[SP2_THREADS / 32];
+__device__ __forceinline__ void sp2_body(const Sp2Args& g, int me, int ctas, double* sm) {
+  __shared__ double red[TILE * 17 * PL], tile[TILE * 17 * PL], sums[2 * SP2_THREADS / 32];
   __shared__ int ok;
-  const int n = g.n, tid = threadIdx.x, ctas = gridDim.x, me = blockIdx.x;
+  const int n = g.n, tid = threadIdx.x, nt = (n + TILE - 1) / TILE, tiles = nt * (nt + 1) / 2;
   unsigned arrivals = 0;
-  double* part[2] = {g.part, g.part + 2 * kMaxCtas};
+  double* part[2] = {g.part, g.part + 2 * kMaxTiles};  // (tr, ||.||_F^2) per tile: the sums do not depend on ctas
 
   // X = (hi - F) / (hi - lo), upper triangle and its mirror
   {
     const double lo = g.b[0], hi = g.b[1], inv = 1.0 / fmax(hi - lo, 1e-300);
-    double tr = 0.0, fro = 0.0;
-    const int64_t n2 = static_cast<int64_t>(n) * n;
-    for (int64_t e = me * static_cast<int64_t>(SP2_THREADS) + tid; e < n2; e += static_cast<int64_t>(ctas) * SP2_THREADS) {
-      const int i = static_cast<int>(e / n), j = static_cast<int>(e - static_cast<int64_t>(i) * n);
-      if (i > j) continue;
-      const int64_t m = static_cast<int64_t>(j) * n + i;
-      const double re = ((i == j ? hi : 0.0) - g.F[e * PL]) * inv, im = PL == 2 && i != j ? -g.F[e * PL + PL - 1] * inv : 0.0;
-      g.X[e * PL] = re;
-      g.X[m * PL] = re;
-      if (PL == 2) {
-        g.X[e * PL + PL - 1] = im;
-        g.X[m * PL + PL - 1] = -im;
+    for (int t = me; t < tiles; t += ctas) {
+      int i0, j0;
+      tile_at(t, nt, i0, j0);
+      const int i = i0 + tid / TILE, j = j0 + tid % TILE;
+      double tr = 0.0, fro = 0.0;
+      if (i < n && j < n && i <= j) {
+        const int64_t e = static_cast<int64_t>(i) * n + j, m = static_cast<int64_t>(j) * n + i;
+        const double re = ((i == j ? hi : 0.0) - g.F[e * PL]) * inv, im = PL == 2 && i != j ? -g.F[e * PL + PL - 1] * inv : 0.0;
+        g.X[e * PL] = re;
+        g.X[m * PL] = re;
+        if (PL == 2) {
+          g.X[e * PL + PL - 1] = im;
+          g.X[m * PL + PL - 1] = -im;
+        }
+        fro = (i == j ? 1.0 : 2.0) * (re * re + im * im);
+        if (i == j) tr = re;
       }
-      fro += (i == j ? 1.0 : 2.0) * (re * re + im * im);
-      if (i == j) tr += re;
-    }
-    tr = cta_sum(tr, sums);
-    fro = cta_sum(fro, sums);
-    if (tid == 0) {
-      part[0][2 * me] = tr;
-      part[0][2 * me + 1] = fro;
+      cta_sum2(tr, fro, sums);
+      if (tid == 0) {
+        part[0][2 * t] = tr;
+        part[0][2 * t + 1] = fro;
+      }
     }
   }
   if (!grid_barrier(g.bar, arrivals += ctas, &ok)) {
@@ -191,29 +230,24 @@ __global__ void __launch_bounds__(SP2_THREADS, 1) sp2_kernel(const Sp2Args g) {
     return;
   }
 
-  const int nt = (n + TILE - 1) / TILE, tiles = nt * (nt + 1) / 2;
   const double tol = fmax(1.0, g.nocc);
   double *cur = g.X, *nxt = g.Y;
   double result = 1.0, t1 = 0.0, t2 = 0.0;
-  for (int step = 0; step < g.max_steps; ++step) {
+  int step = 0;
+  for (; step < g.max_steps; ++step) {
     // tr X and tr X^2 of the matrix about to be squared
     const volatile double* pin = part[step & 1];
-    double a = 0.0, b = 0.0;
-    for (int i = tid; i < ctas; i += SP2_THREADS) {
-      a += pin[2 * i];
-      b += pin[2 * i + 1];
+    t1 = t2 = 0.0;
+    for (int i = tid; i < tiles; i += SP2_THREADS) {
+      t1 += pin[2 * i];
+      t2 += pin[2 * i + 1];
     }
-    t1 = cta_sum(a, sums);
-    t2 = cta_sum(b, sums);
+    cta_sum2(t1, t2, sums);
     const bool square = fabs(t2 - g.nocc) < fabs(2.0 * t1 - t2 - g.nocc);
-    double tr = 0.0, fro = 0.0;
     for (int t = me; t < tiles; t += ctas) {
-      int ti = 0, rest = t;
-      while (rest >= nt - ti) {
-        rest -= nt - ti;
-        ++ti;
-      }
-      const int i0 = ti * TILE, j0 = (ti + rest) * TILE;
+      int i0, j0;
+      tile_at(t, nt, i0, j0);
+      double tr = 0.0, fro = 0.0;
       square_tile<PL>(cur, n, g.kc, i0, j0, sm, red, tile);
       const int r = tid / TILE, c = tid % TILE, i = i0 + r, j = j0 + c;
       if (i < n && j < n && i <= j) {
@@ -233,15 +267,14 @@ __global__ void __launch_bounds__(SP2_THREADS, 1) sp2_kernel(const Sp2Args g) {
           nxt[m + PL - 1] = i == j ? 0.0 : -v[PL - 1];
           sq += v[PL - 1] * v[PL - 1];
         }
-        fro += (i == j ? 1.0 : 2.0) * sq;
-        if (i == j) tr += v[0];
+        fro = (i == j ? 1.0 : 2.0) * sq;
+        if (i == j) tr = v[0];
       }
-    }
-    tr = cta_sum(tr, sums);
-    fro = cta_sum(fro, sums);
-    if (tid == 0) {
-      part[(step + 1) & 1][2 * me] = tr;
-      part[(step + 1) & 1][2 * me + 1] = fro;
+      cta_sum2(tr, fro, sums);
+      if (tid == 0) {
+        part[(step + 1) & 1][2 * t] = tr;
+        part[(step + 1) & 1][2 * t + 1] = fro;
+      }
     }
     if (!grid_barrier(g.bar, arrivals += ctas, &ok)) {
       result = 2.0;
@@ -266,7 +299,25 @@ __global__ void __launch_bounds__(SP2_THREADS, 1) sp2_kernel(const Sp2Args g) {
     g.outcome[0] = result;
     g.outcome[1] = t1;
     g.outcome[2] = t2;
+    g.outcome[3] = step + 1;
   }
+}
+
+template <int PL>
+__global__ void __launch_bounds__(SP2_THREADS, 1) sp2_kernel(const Sp2Args g) {
+  extern __shared__ __align__(16) double sm[];
+  sp2_body<PL>(g, blockIdx.x, gridDim.x, sm);
+}
+
+// Independent complex problems side by side: CTA b works on problem of[b], as one of its ctas from first on.
+struct Sp2Entry {
+  Sp2Args a;
+  int first, ctas;
+};
+__global__ void __launch_bounds__(SP2_THREADS, 1) sp2_group_kernel(const Sp2Entry* tab, const int* of) {
+  extern __shared__ __align__(16) double sm[];
+  const Sp2Entry e = tab[of[blockIdx.x]];
+  sp2_body<2>(e.a, blockIdx.x - e.first, e.ctas, sm);
 }
 
 // ---------------------------------------------------------------- Ritz values
@@ -428,7 +479,78 @@ __global__ void __launch_bounds__(THREADS, 1) ritz_kernel(const double* T, const
 
 }  // namespace
 
-int64_t sp2_scratch_doubles() { return 4 * kMaxCtas + 32; }
+namespace {
+
+Sp2Args make_args(const Sp2Problem& q, bool cplx, bool sure, int max_steps) {
+  const int PL = cplx ? 2 : 1;
+  Sp2Args g{};
+  g.F = q.F;
+  g.b = q.b;
+  g.X = q.X;
+  g.Y = q.Y;
+  g.part = q.scratch;
+  g.bar = reinterpret_cast<unsigned*>(q.scratch + 4 * kMaxTiles);
+  g.outcome = q.outcome;
+  g.nocc = q.nocc;
+  g.n = static_cast<int>(q.n);
+  g.max_steps = max_steps;
+  g.sure = sure;
+  const int kfit = kSp2Smem / static_cast<int>(sizeof(double)) / (2 * TILE * PL) - 4;
+  g.kc = std::min<int>(static_cast<int>(round_up(q.n, 8)), kfit / 8 * 8);
+  return g;
+}
+int smem_of(const Sp2Args& g, int PL) { return static_cast<int>(sizeof(double)) * 2 * TILE * PL * (g.kc + 4); }
+int tiles_of(int64_t n) {
+  const int nt = static_cast<int>((n + TILE - 1) / TILE);
+  return nt * (nt + 1) / 2;
+}
+
+}  // namespace
+
+int64_t sp2_scratch_doubles() { return 4 * kMaxTiles + 32; }
+
+void sp2_run_group(const Sp2Problem* p, int count, const std::function<const void*(const void*, size_t)>& put, cudaStream_t s) {
+  static std::atomic<bool> attr[kMaxDevices];
+  once_per_device(attr, [] {
+    RR_CUDA(cudaFuncSetAttribute(sp2_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSp2Smem));
+  });
+  // at most half as many problems a launch as CTAs fit the GPU at once; CTAs in proportion to a step's work
+  for (int p0 = 0; p0 < count;) {
+    int smem = 0, many = 0, per_sm = 0, room = 0;
+    std::vector<Sp2Entry> tab;
+    std::vector<double> work;
+    double all = 0.0;
+    while (p0 + many < count) {
+      Sp2Entry e{};
+      e.a = make_args(p[p0 + many], true, true, 120);
+      const int need = std::max(smem, smem_of(e.a, 2));
+      RR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sp2_group_kernel, SP2_THREADS, need));
+      const int fits = std::min(per_sm * sm_count_current(), kMaxGroupCtas);
+      if (many > 0 && many + 1 > fits / 2) break;
+      room = fits;
+      smem = need;
+      tab.push_back(e);
+      work.push_back(static_cast<double>(tiles_of(e.a.n)) * e.a.n);
+      all += work.back();
+      ++many;
+    }
+    std::vector<int> of;
+    for (int i = 0; i < many; ++i) {
+      const int share = static_cast<int>((room - many) * (work[i] / all));
+      tab[i].first = static_cast<int>(of.size());
+      tab[i].ctas = std::max(1, std::min(1 + share, tiles_of(tab[i].a.n)));
+      of.insert(of.end(), tab[i].ctas, i);
+      RR_CUDA(cudaMemsetAsync(tab[i].a.bar, 0, 2 * sizeof(unsigned), s));
+    }
+    const Sp2Entry* dt = static_cast<const Sp2Entry*>(put(tab.data(), sizeof(Sp2Entry) * tab.size()));
+    const int* dof = static_cast<const int*>(put(of.data(), sizeof(int) * of.size()));
+    void* args[] = {&dt, &dof};
+    RR_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(sp2_group_kernel), dim3(static_cast<unsigned>(of.size())),
+                                        dim3(SP2_THREADS), args, smem, s));
+    RR_LAUNCH_CHECK();
+    p0 += many;
+  }
+}
 
 void sp2_run(const double* F, int64_t n, double nocc, bool cplx, const double* b, bool sure, int max_steps, double* X, double* Y,
              double* scratch, double* outcome, cudaStream_t s) {
@@ -438,23 +560,8 @@ void sp2_run(const double* F, int64_t n, double nocc, bool cplx, const double* b
     RR_CUDA(cudaFuncSetAttribute(sp2_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSp2Smem));
     RR_CUDA(cudaFuncSetAttribute(sp2_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSp2Smem));
   });
-  Sp2Args g{};
-  g.F = F;
-  g.b = b;
-  g.X = X;
-  g.Y = Y;
-  g.part = scratch;
-  g.bar = reinterpret_cast<unsigned*>(scratch + 4 * kMaxCtas);
-  g.outcome = outcome;
-  g.nocc = nocc;
-  g.n = static_cast<int>(n);
-  g.max_steps = max_steps;
-  g.sure = sure;
-  const int kfit = kSp2Smem / static_cast<int>(sizeof(double)) / (2 * TILE * PL) - 4;
-  g.kc = std::min<int>(static_cast<int>(round_up(n, 8)), kfit / 8 * 8);
-  const int smem = static_cast<int>(sizeof(double)) * 2 * TILE * PL * (g.kc + 4);
-  const int nt = static_cast<int>((n + TILE - 1) / TILE), tiles = nt * (nt + 1) / 2;
-  const int grid = std::max(1, std::min({tiles, sm_count_current(), kMaxCtas}));
+  Sp2Args g = make_args(Sp2Problem{F, b, X, Y, scratch, outcome, nocc, n}, cplx, sure, max_steps);
+  const int smem = smem_of(g, PL), grid = std::max(1, std::min(tiles_of(n), sm_count_current()));
   RR_CUDA(cudaMemsetAsync(g.bar, 0, 2 * sizeof(unsigned), s));
   void* args[] = {&g};
   RR_CUDA(cudaLaunchCooperativeKernel(cplx ? reinterpret_cast<const void*>(sp2_kernel<2>) : reinterpret_cast<const void*>(sp2_kernel<1>),

@@ -1,23 +1,35 @@
 // One-launch forms of the density step's purification (sp2.cu).
 #pragma once
 
+#include <functional>
+
 #include "rr_common.cuh"
 
 namespace rr {
 
-// Largest n the one-launch purification takes.  SCF loop, product + step launches / one launch, ms: n = 48 6.4 / 3.4, 160 6.9 /
-// 5.4, 240 9.2 / 7.8, 400 16.5 / 15.5; complex n = 232 4.0 / 3.3, 314 5.1 / 4.5.  Beyond that a step's products fill the GPU by themselves.
+// Largest n the one-launch purification takes.  SCF loop, product + step launches / one launch, ms: n = 48 6.4 / 2.7, 160 6.9 /
+// 5.0, 240 9.2 / 7.1, 400 16.5 / 14.8; complex n = 232 4.0 / 3.3, 314 5.1 / 4.2.  Beyond that a step's products fill the GPU by themselves.
 constexpr int64_t kSp2MaxReal = 512, kSp2MaxComplex = 400;
 
 // Doubles of scratch sp2_run needs besides X's second buffer.
 int64_t sp2_scratch_doubles();
 
 // SP2 purification of the Hermitian F (n x n): X <- the projector onto its lowest `nocc` eigenvectors, from the spectral
-// interval b = [lo, hi] (device; sure: it holds the spectrum for certain); Y: a second n x n buffer; scratch: sp2_scratch_doubles().  outcome (device, 3 doubles): [0]
+// interval b = [lo, hi] (device; sure: it holds the spectrum for certain); Y: a second n x n buffer; scratch: sp2_scratch_doubles().  outcome (device, 4 doubles): [0]
 // = 0 converged, 1 the interval missed part of the spectrum (or max_steps passed), 2 a grid barrier expired; [1], [2] = tr X and
-// tr X^2 of the last step.
+// tr X^2 of the last step; [3] = steps.
 void sp2_run(const double* F, int64_t n, double nocc, bool cplx, const double* b, bool sure, int max_steps, double* X,
              double* Y, double* scratch, double* outcome, cudaStream_t s);
+
+// The same for complex problems side by side, each on its own group of CTAs with its own barrier (b holds the spectrum,
+// at most 120 steps).  put copies a table to the device for launches on s.
+struct Sp2Problem {
+  const double *F, *b;
+  double *X, *Y, *scratch, *outcome;
+  double nocc;
+  int64_t n;
+};
+void sp2_run_group(const Sp2Problem* p, int count, const std::function<const void*(const void*, size_t)>& put, cudaStream_t s);
 
 // b = [lo, hi] narrowed to the extreme eigenvalues of T y = theta M y (k x k, k = 32, full Hermitian, M positive
 // definite), widened by 10 % of their distance on both sides; unchanged when M is not positive definite.
