@@ -55,10 +55,22 @@ struct GCfg {
   static constexpr int TMEM_COLS = 128;
 };
 
-__global__ void __launch_bounds__(128, 1)
-    umma_gemm_kernel(const __grid_constant__ CUtensorMap mapA_hi, const __grid_constant__ CUtensorMap mapA_lo,
-                     const __grid_constant__ CUtensorMap mapB_hi, const __grid_constant__ CUtensorMap mapB_lo,
-                     const GParams p) {
+// Up to kGProds products in one launch: CTA first[i] + split * tiles + tile works on product i.  One launch per product
+// left most SMs idle at its end and in its set-up: X2C nl = 131, 54 electrons, six products of 131 x 131 x 28 k: 163 us
+// one by one, 142 in one launch (the K ranges, and so the FP32 sums, are the same).
+constexpr int kGProds = 6;
+struct GBatch {
+  CUtensorMap map[kGProds][4];  // A hi, A lo, B hi, B lo
+  GParams p[kGProds];
+  int first[kGProds + 1], count;
+};
+
+__global__ void __launch_bounds__(128, 1) umma_gemm_kernel(const __grid_constant__ GBatch batch) {
+  int prod = 0;
+  while (prod + 1 < batch.count && static_cast<int>(blockIdx.x) >= batch.first[prod + 1]) ++prod;
+  const GParams& p = batch.p[prod];
+  const CUtensorMap &mapA_hi = batch.map[prod][0], &mapA_lo = batch.map[prod][1], &mapB_hi = batch.map[prod][2],
+                    &mapB_lo = batch.map[prod][3];
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + G_STAGES * GCfg::STAGE);
@@ -67,7 +79,7 @@ __global__ void __launch_bounds__(128, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  const int tile = blockIdx.x, split = blockIdx.y;
+  const int local = static_cast<int>(blockIdx.x) - batch.first[prod], split = local / p.tiles, tile = local - split * p.tiles;
   int tm, tn;
   if (p.upper) {  // tile -> (tm, tn), tm <= tn, row-major over the upper triangle
     tm = 0;
@@ -160,46 +172,64 @@ __global__ void __launch_bounds__(128, 1)
   if (warp == 0) tmem_dealloc(tmem, GCfg::TMEM_COLS);
 }
 
-// Fixed-order reduction of the split-K partial tiles of one exchange block, scattered into K:
+// Fixed-order reduction of the split-K partial tiles of exchange blocks (blockIdx.y), scattered into K:
 // value(a, b) = sum_s work[s][tile(a, b)][a % 128][b % 128] (real part from wre, imaginary part from
 // wim when given).  For an upper-tile block the lower triangle takes the mirrored value, with the
 // imaginary part negated (Hermitian).  K entry (of + a, ou + b) receives the value; with `both` the
 // entry (ou + b, of + a) receives its conjugate.  Complex K is interleaved.
-__global__ void umma_place_kernel(const float* wre, const float* wim, int splits, int tiles, int ntn, int upper, int M,
-                                  int N, double* K, int64_t ldk, int64_t of, int64_t ou, int both, int accumulate,
-                                  int cplx) {
-  const int64_t tile_sz = static_cast<int64_t>(BM) * GBN;
-  for (int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; idx < static_cast<int64_t>(M) * N;
-       idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int a = static_cast<int>(idx / N), b = static_cast<int>(idx % N);
-    int i = a, j = b;
-    double sim = 1.0;
-    if (upper && a > b) { i = b; j = a; sim = -1.0; }
-    const int tm = i / BM, tn = j / GBN;
-    const int t = upper ? tm * ntn - tm * (tm - 1) / 2 + (tn - tm) : tm * ntn + tn;
-    const int64_t off = static_cast<int64_t>(t) * tile_sz + static_cast<int64_t>(i - tm * BM) * GBN + (j - tn * GBN);
+// Bound: reading the partials once.  A CTA takes 32 columns of a row, its eight warps every eighth split (their sums are
+// added in the order of the warps); an upper-tile block is read from its upper triangle only.  With one thread an element walking
+// all 99 splits: 24 us a block, three blocks one after the other, at the sizes above; now 24 us for the three.
+struct PlaceBlock {
+  const float *wre, *wim;
+  int splits, tiles, ntn, upper, M, N, both;
+  int64_t of, ou;
+};
+struct PlaceList {
+  PlaceBlock b[kGProds];
+};
+constexpr int kPlaceWarps = 8;
+__global__ void __launch_bounds__(32 * kPlaceWarps) umma_place_kernel(const __grid_constant__ PlaceList list, double* K, int64_t ldk,
+                                                                      int accumulate, int cplx) {
+  __shared__ double sre[kPlaceWarps][32], sim[kPlaceWarps][32];
+  const PlaceBlock& q = list.b[blockIdx.y];
+  const int64_t tile_sz = static_cast<int64_t>(BM) * GBN, step = static_cast<int64_t>(q.tiles) * tile_sz;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int groups = (q.N + 31) / 32;
+  for (int64_t item = blockIdx.x; item < static_cast<int64_t>(q.M) * groups; item += gridDim.x) {
+    const int a = static_cast<int>(item / groups), c0 = static_cast<int>(item % groups) * 32, b = c0 + lane;
+    if (q.upper && c0 + 31 < a) continue;  // (uniform) below the diagonal: written with its mirror
+    const bool live = b < q.N && !(q.upper && b < a);
     double re = 0.0, im = 0.0;
-    for (int sp = 0; sp < splits; ++sp) re += static_cast<double>(wre[static_cast<int64_t>(sp) * tiles * tile_sz + off]);
-    if (wim)
-      for (int sp = 0; sp < splits; ++sp) im += static_cast<double>(wim[static_cast<int64_t>(sp) * tiles * tile_sz + off]);
-    im = upper && a == b ? 0.0 : im * sim;  // a Hermitian block has a real diagonal
-    if (cplx) {
-      double* k = K + ((of + a) * ldk + ou + b) * 2;
-      k[0] = accumulate ? k[0] + re : re;
-      k[1] = accumulate ? k[1] + im : im;
-      if (both) {
-        double* kt = K + ((ou + b) * ldk + of + a) * 2;
-        kt[0] = accumulate ? kt[0] + re : re;
-        kt[1] = accumulate ? kt[1] - im : -im;
-      }
-    } else {
-      double* k = K + (of + a) * ldk + ou + b;
-      *k = accumulate ? *k + re : re;
-      if (both) {
-        double* kt = K + (ou + b) * ldk + of + a;
-        *kt = accumulate ? *kt + re : re;
+    if (live) {
+      const int tm = a / BM, tn = b / GBN;
+      const int t = q.upper ? tm * q.ntn - tm * (tm - 1) / 2 + (tn - tm) : tm * q.ntn + tn;
+      const int64_t off = t * tile_sz + static_cast<int64_t>(a - tm * BM) * GBN + (b - tn * GBN);
+#pragma unroll 4
+      for (int sp = w; sp < q.splits; sp += kPlaceWarps) {
+        re += static_cast<double>(q.wre[sp * step + off]);
+        if (q.wim) im += static_cast<double>(q.wim[sp * step + off]);
       }
     }
+    sre[w][lane] = re;
+    sim[w][lane] = im;
+    __syncthreads();
+    if (w == 0 && live) {
+      for (int i = 1; i < kPlaceWarps; ++i) {
+        re += sre[i][lane];
+        im += sim[i][lane];
+      }
+      auto put = [&](int64_t r, int64_t c, double x, double y) {
+        double* k = K + (r * ldk + c) * (cplx ? 2 : 1);
+        k[0] = accumulate ? k[0] + x : x;
+        if (cplx) k[1] = accumulate ? k[1] + y : y;
+      };
+      if (q.upper && a == b) im = 0.0;  // a Hermitian block has a real diagonal
+      put(q.of + a, q.ou + b, re, im);
+      if (q.upper && a != b) put(q.of + b, q.ou + a, re, -im);
+      if (q.both) put(q.ou + b, q.of + a, re, -im);
+    }
+    __syncthreads();
   }
 }
 
@@ -589,20 +619,21 @@ BlockPlan plan_block(int64_t M, int64_t N, int64_t kt, bool upper) {
   return b;
 }
 
-// K-contiguous product A (M x kt) . B (N x kt)^T of two split planes (row pitch ldt) into FP32
-// partial tiles.
-void launch_gemm(const BlockPlan& bp, const uint16_t* a_hi, const uint16_t* a_lo, int64_t M, const uint16_t* b_hi,
-                 const uint16_t* b_lo, int64_t N, int64_t kt, int64_t ldt, float* work, int* err, cudaStream_t s) {
+// Adds the K-contiguous product A (M x kt) . B (N x kt)^T of two split planes (row pitch ldt) into FP32 partial
+// tiles to a launch.
+void add_product(GBatch& g, const BlockPlan& bp, const uint16_t* a_hi, const uint16_t* a_lo, int64_t M, const uint16_t* b_hi,
+                 const uint16_t* b_lo, int64_t N, int64_t kt, int64_t ldt, float* work, int* err) {
   uint64_t dimsA[2] = {static_cast<uint64_t>(kt), static_cast<uint64_t>(M)};
   uint64_t dimsB[2] = {static_cast<uint64_t>(kt), static_cast<uint64_t>(N)};
   uint64_t str[1] = {static_cast<uint64_t>(ldt) * 2};
   uint32_t boxA[2] = {BK, BM};
   uint32_t boxB[2] = {BK, GBN};
-  const CUtensorMap mah = make_map(a_hi, 2, dimsA, str, boxA);
-  const CUtensorMap mal = make_map(a_lo, 2, dimsA, str, boxA);
-  const CUtensorMap mbh = make_map(b_hi, 2, dimsB, str, boxB);
-  const CUtensorMap mbl = make_map(b_lo, 2, dimsB, str, boxB);
-  GParams p{};
+  const int i = g.count++;
+  g.map[i][0] = make_map(a_hi, 2, dimsA, str, boxA);
+  g.map[i][1] = make_map(a_lo, 2, dimsA, str, boxA);
+  g.map[i][2] = make_map(b_hi, 2, dimsB, str, boxB);
+  g.map[i][3] = make_map(b_lo, 2, dimsB, str, boxB);
+  GParams& p = g.p[i];
   p.kblocks = bp.kblocks;
   p.splits = bp.splits;
   p.tiles = bp.tiles;
@@ -610,12 +641,15 @@ void launch_gemm(const BlockPlan& bp, const uint16_t* a_hi, const uint16_t* a_lo
   p.upper = bp.upper ? 1 : 0;
   p.work = work;
   p.err = err;
+  g.first[i + 1] = g.first[i] + bp.tiles * bp.splits;
+}
+
+void launch_products(const GBatch& g, cudaStream_t s) {
   static std::atomic<bool> attr[kMaxDevices];
   once_per_device(attr, [] {
     RR_CUDA(cudaFuncSetAttribute(umma_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GCfg::SMEM));
   });
-  umma_gemm_kernel<<<dim3(static_cast<unsigned>(bp.tiles), static_cast<unsigned>(bp.splits)), 128, GCfg::SMEM, s>>>(
-      mah, mal, mbh, mbl, p);
+  umma_gemm_kernel<<<static_cast<unsigned>(g.first[g.count]), 128, GCfg::SMEM, s>>>(g);
   RR_LAUNCH_CHECK();
 }
 
@@ -727,9 +761,15 @@ void mixed_exchange_general(const MixedOperands* ops, MixedScratch& scr, const E
     pl_off[f] = pl_sz;
     pl_sz += round_up(planes * fl.fs[f] * ldt, 128);
   }
-  for (const Blk& b : blocks) {
-    const BlockPlan bp = plan_block(fl.fs[b.f], fl.fs[b.u], kt, b.upper);
-    work_sz = std::max<int64_t>(work_sz, pl * static_cast<int64_t>(bp.splits) * bp.tiles * BM * GBN);
+  // Blocks of one launch: their real (and imaginary) products side by side in the partials.
+  const size_t per_launch = static_cast<size_t>(kGProds / pl);
+  for (size_t b0 = 0; b0 < blocks.size(); b0 += per_launch) {
+    int64_t sz = 0;
+    for (size_t k = b0; k < std::min(blocks.size(), b0 + per_launch); ++k) {
+      const BlockPlan bp = plan_block(fl.fs[blocks[k].f], fl.fs[blocks[k].u], kt, blocks[k].upper);
+      sz += pl * static_cast<int64_t>(bp.splits) * bp.tiles * BM * GBN;
+    }
+    work_sz = std::max(work_sz, sz);
   }
   scr.coef_hi.ensure(static_cast<size_t>(coef_sz));
   scr.coef_lo.ensure(static_cast<size_t>(coef_sz));
@@ -787,21 +827,31 @@ void mixed_exchange_general(const MixedOperands* ops, MixedScratch& scr, const E
       std::memcpy(e.sgn, sgn, sizeof(sgn));
       launch_ht(mo, scr.coef_hi.p, scr.coef_lo.p, rows, e, err, s);
     }
-    for (const Blk& b : blocks) {
-      const BlockPlan bp = plan_block(fl.fs[b.f], fl.fs[b.u], kt, b.upper);
-      const int64_t part = static_cast<int64_t>(bp.splits) * bp.tiles * BM * GBN;
-      float* wre = scr.work.p;
-      float* wim = cplx ? scr.work.p + part : nullptr;
-      launch_gemm(bp, plane(scr.pl_hi.p, b.f, 0), plane(scr.pl_lo.p, b.f, 0), fl.fs[b.f], plane(scr.pl_hi.p, b.u, pre),
-                  plane(scr.pl_lo.p, b.u, pre), fl.fs[b.u], kt, ldt, wre, err, s);
-      if (cplx)
-        launch_gemm(bp, plane(scr.pl_hi.p, b.f, 0), plane(scr.pl_lo.p, b.f, 0), fl.fs[b.f],
-                    plane(scr.pl_hi.p, b.u, planes - 1), plane(scr.pl_lo.p, b.u, planes - 1), fl.fs[b.u], kt, ldt,
-                    wim, err, s);
-      const int both = !incr && b.f != b.u ? 1 : 0;
-      umma_place_kernel<<<grid_for(fl.fs[b.f] * fl.fs[b.u]), 256, 0, s>>>(
-          wre, wim, bp.splits, bp.tiles, bp.ntn, bp.upper ? 1 : 0, static_cast<int>(fl.fs[b.f]),
-          static_cast<int>(fl.fs[b.u]), target, ldk, fl.off[b.f], fl.off[b.u], both, 1, cplx ? 1 : 0);
+    for (size_t b0 = 0; b0 < blocks.size(); b0 += per_launch) {
+      GBatch gb{};
+      PlaceList place{};
+      float* w = scr.work.p;
+      int64_t most = 1;
+      unsigned nblocks = 0;
+      for (size_t k = b0; k < std::min(blocks.size(), b0 + per_launch); ++k) {
+        const Blk& b = blocks[k];
+        const BlockPlan bp = plan_block(fl.fs[b.f], fl.fs[b.u], kt, b.upper);
+        const int64_t part = static_cast<int64_t>(bp.splits) * bp.tiles * BM * GBN;
+        float* wre = w;
+        float* wim = cplx ? w + part : nullptr;
+        w += pl * part;
+        add_product(gb, bp, plane(scr.pl_hi.p, b.f, 0), plane(scr.pl_lo.p, b.f, 0), fl.fs[b.f], plane(scr.pl_hi.p, b.u, pre),
+                    plane(scr.pl_lo.p, b.u, pre), fl.fs[b.u], kt, ldt, wre, err);
+        if (cplx)
+          add_product(gb, bp, plane(scr.pl_hi.p, b.f, 0), plane(scr.pl_lo.p, b.f, 0), fl.fs[b.f],
+                      plane(scr.pl_hi.p, b.u, planes - 1), plane(scr.pl_lo.p, b.u, planes - 1), fl.fs[b.u], kt, ldt, wim, err);
+        place.b[nblocks++] = PlaceBlock{wre, wim, bp.splits, bp.tiles, bp.ntn, bp.upper ? 1 : 0, static_cast<int>(fl.fs[b.f]),
+                                        static_cast<int>(fl.fs[b.u]), !incr && b.f != b.u ? 1 : 0, fl.off[b.f], fl.off[b.u]};
+        most = std::max(most, fl.fs[b.f] * ((fl.fs[b.u] + 31) / 32));
+      }
+      launch_products(gb, s);
+      umma_place_kernel<<<dim3(static_cast<unsigned>(std::min<int64_t>(most, 8LL * sm_count())), nblocks), 32 * kPlaceWarps, 0, s>>>(
+          place, target, ldk, 1, cplx ? 1 : 0);
       RR_LAUNCH_CHECK();
     }
   }
