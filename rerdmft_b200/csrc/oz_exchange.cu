@@ -368,11 +368,30 @@ int64_t mo_range(int64_t naux, int64_t bytes_per_row) {
   return std::max<int64_t>(1, std::min<int64_t>(naux, (96LL << 20) / std::max<int64_t>(bytes_per_row, 1)));
 }
 
+// A range of at most `most` aux rows whose two launches (n rows an aux row, n columns) fill their last round of tiles: a CTA
+// walks whole tiles, and 75 rows of n = 400 are 1645 of them, 11.1 a CTA, 74 rows 1624, 10.97.  n = 400, naux = 1600: 8.0 ->
+// 7.6 ms.  (Not for the four-component transform: its five launches of different shapes gain nothing, 5.13 / 5.17 ms.)
+int64_t mo_even_range(int64_t naux, int64_t most, int64_t n) {
+  if (most >= naux) return most;
+  const int64_t sms = sm_count_current();
+  int64_t best = most;
+  double best_cost = 0.0;
+  for (int64_t pc = std::max<int64_t>(1, most - most / 4); pc <= most; ++pc) {
+    const int64_t tiles = (pc * n + oz::kBM - 1) / oz::kBM * ((n + oz::kBN - 1) / oz::kBN);
+    const double cost = static_cast<double>((tiles + sms - 1) / sms) / static_cast<double>(pc);
+    if (best_cost == 0.0 || cost <= best_cost) {
+      best_cost = cost;
+      best = pc;
+    }
+  }
+  return best;
+}
+
 // out[P] = C^T B^P C for device C (n x n).
 bool mo_real(const double* B, int64_t pitch, int64_t n, int64_t naux, const double* cscale, const double* pnorm, const uint8_t* resident,
              const double* C, double* out, Carve& c, int* err, cudaStream_t s) {
   const int64_t ncp = round_up(n, 16), per_row = kDigits * n * round_up(n, oz::kBK);
-  const int64_t pc = mo_range(naux, resident ? per_row : 2 * per_row);
+  const int64_t pc = mo_even_range(naux, mo_range(naux, resident ? per_row : 2 * per_row), n);
   const int64_t o_coef = c.take(coef_bytes(ncp, n)), o_cs = c.take(8 * ncp), o_norm = c.take(8 * ncp),
                 o_row = c.take(16 * naux * n), o_y = c.take(left_bytes(pc * n, n)),
                 o_b = c.take(resident ? 0 : left_bytes(pc * n, n));
