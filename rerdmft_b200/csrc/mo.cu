@@ -153,13 +153,21 @@ __global__ void subblock_kernel(double* out, const double* B, int64_t naux, int6
   }
 }
 
-// Block-diagonal (alpha, beta) embedding of a spatial tensor (src/NON_REL/NonRelSpinRiMoEri.h:77).
-__global__ void embed_kernel(double* out, const double* B, int64_t naux, int64_t n) {
-  const int64_t m = 2 * n;
-  for (int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; idx < naux * m * m;
-       idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t P = idx / (m * m), r = idx % (m * m), i = r / m, j = r % m;
-    out[idx] = (i / n == j / n) ? B[P * n * n + (i % n) * n + (j % n)] : 0.0;
+// Block-diagonal (alpha, beta) embedding of a spatial tensor (src/NON_REL/NonRelSpinRiMoEri.h:77), a warp per output row.
+// Bound: its 8 bytes written (and a quarter read) per element; with a thread per element four 64-bit divisions each were:
+// n = 120, naux = 480 (221 MB) 174 us, now 75.
+__global__ void __launch_bounds__(256) embed_kernel(double* out, const double* B, int64_t naux, int64_t n) {
+  const int64_t m = 2 * n, rows = naux * m;
+  const int lane = threadIdx.x & 31;
+  for (int64_t r = blockIdx.x * 8LL + (threadIdx.x >> 5); r < rows; r += gridDim.x * 8LL) {
+    const int64_t P = r / m, i = r - P * m, shift = i < n ? 0 : n;
+    const double* src = B + (P * n + i - shift) * n;
+    double* dst = out + r * m;
+#pragma unroll 4
+    for (int64_t j = lane; j < m; j += 32) {
+      const int64_t jj = j - shift;
+      dst[j] = jj >= 0 && jj < n ? src[jj] : 0.0;
+    }
   }
 }
 
@@ -188,46 +196,94 @@ __global__ void spin_average_kernel(const double* U, int64_t n, double* u, doubl
 
 // Generalized-Fock pieces (src/Hessian_opt/RiGemmFock.cpp:92-157).
 // F(p,q) = occ_q h(q,p) + sum_P B(P,q,p) W(P,q)
+// A CTA takes 32 p of one q, its eight warps every eighth P (sums added in the order of the warps).  Bound: reading B once; with one
+// thread an element walking all P: d = 240, naux = 480 146 us, now 68.
 template <int PL>
-__global__ void hx_f0f1_kernel(const double* B, const double* W, const double* h, const double* occ, int64_t naux,
-                               int64_t n, double* F) {
-  for (int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; idx < n * n;
-       idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t q = idx / n, p = idx % n;  // p fastest: B(P,q,p) reads coalesced
+__global__ void __launch_bounds__(256) hx_f0f1_kernel(const double* B, const double* W, const double* h, const double* occ, int64_t naux,
+                                                      int64_t n, double* F) {
+  __shared__ double part[8][32][PL];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t groups = (n + 31) / 32;
+  for (int64_t item = blockIdx.x; item < n * groups; item += gridDim.x) {
+    const int64_t q = item / groups, p = (item - q * groups) * 32 + lane;
     double sr = 0.0, si = 0.0;
-    for (int64_t P = 0; P < naux; ++P) {
-      const double br = B[(P * n * n + q * n + p) * PL], bi = PL == 2 ? B[(P * n * n + q * n + p) * PL + 1] : 0.0;
-      const double wr = W[(P * n + q) * PL], wi = PL == 2 ? W[(P * n + q) * PL + 1] : 0.0;
-      sr += br * wr - bi * wi;
-      si += br * wi + bi * wr;
+    if (p < n) {
+#pragma unroll 4
+      for (int64_t P = w; P < naux; P += 8) {
+        const double br = B[(P * n * n + q * n + p) * PL], bi = PL == 2 ? B[(P * n * n + q * n + p) * PL + PL - 1] : 0.0;
+        const double wr = W[(P * n + q) * PL], wi = PL == 2 ? W[(P * n + q) * PL + PL - 1] : 0.0;
+        sr += br * wr - bi * wi;
+        si += br * wi + bi * wr;
+      }
     }
-    const double o = occ[q];
-    double* f = F + (p * n + q) * PL;
-    f[0] = o * h[(q * n + p) * PL] + sr;
-    if (PL == 2) f[1] = o * h[(q * n + p) * PL + 1] + si;
+    part[w][lane][0] = sr;
+    if (PL == 2) part[w][lane][PL - 1] = si;
+    __syncthreads();
+    if (w == 0 && p < n) {
+      for (int g = 1; g < 8; ++g) {
+        sr += part[g][lane][0];
+        if (PL == 2) si += part[g][lane][PL - 1];
+      }
+      const double o = occ[q];
+      double* f = F + (p * n + q) * PL;
+      f[0] = o * h[(q * n + p) * PL] + sr;
+      if (PL == 2) f[1] = o * h[(q * n + p) * PL + 1] + si;
+    }
+    __syncthreads();
   }
 }
 
 // Y(P,t,q) = -x2(q,t) B(P,q,t) [+ 2 (l1(st,qbar) + l2(st,q)) B(P,st,qbar), st = pair_of[t]] for a
 // chunk of aux rows [P0, P0 + pc).
+// A CTA takes a 32 x 32 tile (t, q) of a stretch of aux rows: the coefficients and gather offsets are read and formed once, each
+// B tile is transposed through shared memory.  Bound: B read twice, Y written once; with a thread per element four 64-bit
+// divisions, three coefficient reads and a column-wise read of B each: d = 240, naux = 480 270 us, now 139.
 template <int PL>
-__global__ void hx_y_kernel(const double* B, int64_t P0, int64_t pc, int64_t n, const double* x2, const int64_t* pair_of,
-                            const double* l1, const double* l2, double* Y) {
-  for (int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; idx < pc * n * n;
-       idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t pl = idx / (n * n), r = idx % (n * n), t = r / n, q = r % n;
-    const double* bp = B + (P0 + pl) * n * n * PL;
-    const double c = -x2[q * n + t];
-    double vr = c * bp[(q * n + t) * PL];
-    double vi = PL == 2 ? c * bp[(q * n + t) * PL + 1] : 0.0;
-    if (pair_of) {
+__global__ void __launch_bounds__(256) hx_y_kernel(const double* B, int64_t P0, int64_t pc, int64_t n, const double* x2, const int64_t* pair_of,
+                                                   const double* l1, const double* l2, double* Y) {
+  __shared__ double tile[PL][32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t nt = (n + 31) / 32, t0 = blockIdx.x / nt * 32, q0 = blockIdx.x % nt * 32, q = q0 + tx;
+  double c[4], w[4] = {0.0, 0.0, 0.0, 0.0};
+  int64_t at[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int64_t t = t0 + ty + 8 * k;
+    const bool in = t < n && q < n;
+    c[k] = in ? -x2[q * n + t] : 0.0;
+    if (in && pair_of) {
       const int64_t st = pair_of[t], qb = pair_of[q];
-      const double w = 2.0 * (l1[st * n + qb] + l2[st * n + q]);
-      vr += w * bp[(st * n + qb) * PL];
-      if (PL == 2) vi += w * bp[(st * n + qb) * PL + 1];
+      w[k] = 2.0 * (l1[st * n + qb] + l2[st * n + q]);
+      at[k] = st * n + qb;
     }
-    Y[idx * PL] = vr;
-    if (PL == 2) Y[idx * PL + 1] = vi;
+  }
+  for (int64_t pl = blockIdx.y; pl < pc; pl += gridDim.y) {
+    const double* bp = B + (P0 + pl) * n * n * PL;
+    double g[4][PL];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int64_t row = q0 + ty + 8 * k, col = t0 + tx;
+      const bool in = row < n && col < n;
+#pragma unroll
+      for (int z = 0; z < PL; ++z) {
+        g[k][z] = pair_of ? bp[at[k] * PL + z] : 0.0;
+        tile[z][ty + 8 * k][tx] = in ? bp[(row * n + col) * PL + z] : 0.0;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int64_t t = t0 + ty + 8 * k;
+      if (t < n && q < n) {
+#pragma unroll
+        for (int z = 0; z < PL; ++z) {
+          double v = c[k] * tile[z][tx][ty + 8 * k];
+          if (pair_of) v += w[k] * g[k][z];
+          Y[((pl * n + t) * n + q) * PL + z] = v;
+        }
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -522,8 +578,9 @@ void hx_fock_core(rr_mo_store* m, const double* Bt, int64_t d, int PL, const dou
   w.M = naux; w.N = d; w.K = d;
   w.A = bd; w.lda = d; w.B = h2use; w.ldb = d; w.C = W; w.ldc = d;
   gemm(w, s);
-  if (cplx) hx_f0f1_kernel<2><<<blocks_for(d * d), 256, 0, s>>>(Bt, W, h, occ, naux, d, F);
-  else hx_f0f1_kernel<1><<<blocks_for(d * d), 256, 0, s>>>(Bt, W, h, occ, naux, d, F);
+  const int fgrid = static_cast<int>(std::min<int64_t>(d * ((d + 31) / 32), 2368));
+  if (cplx) hx_f0f1_kernel<2><<<fgrid, 256, 0, s>>>(Bt, W, h, occ, naux, d, F);
+  else hx_f0f1_kernel<1><<<fgrid, 256, 0, s>>>(Bt, W, h, occ, naux, d, F);
   RR_LAUNCH_CHECK();
   // G = sum over aux chunks of B_view^T Y, B_view = (pc*d) x d rows (P,t), Y likewise
   const int64_t pc = chunk_rows(naux, PL * d * d);
@@ -531,8 +588,10 @@ void hx_fock_core(rr_mo_store* m, const double* Bt, int64_t d, int PL, const dou
   bool first = true;
   for (int64_t P0 = 0; P0 < naux; P0 += pc) {
     const int64_t cnt = std::min(pc, naux - P0);
-    if (cplx) hx_y_kernel<2><<<blocks_for(cnt * d * d), 256, 0, s>>>(Bt, P0, cnt, d, x2, pair_of, l1, l2, m->T.p);
-    else hx_y_kernel<1><<<blocks_for(cnt * d * d), 256, 0, s>>>(Bt, P0, cnt, d, x2, pair_of, l1, l2, m->T.p);
+    const int64_t tiles = ((d + 31) / 32) * ((d + 31) / 32);
+    const dim3 ygrid(static_cast<unsigned>(tiles), static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(cnt, 2368 / tiles))));
+    if (cplx) hx_y_kernel<2><<<ygrid, 256, 0, s>>>(Bt, P0, cnt, d, x2, pair_of, l1, l2, m->T.p);
+    else hx_y_kernel<1><<<ygrid, 256, 0, s>>>(Bt, P0, cnt, d, x2, pair_of, l1, l2, m->T.p);
     RR_LAUNCH_CHECK();
     GemmDesc g;
     g.cplx = cplx;
