@@ -235,21 +235,23 @@ __global__ void __launch_bounds__(256) hx_f0f1_kernel(const double* B, const dou
 
 // Y(P,t,q) = -x2(q,t) B(P,q,t) [+ 2 (l1(st,qbar) + l2(st,q)) B(P,st,qbar), st = pair_of[t]] for a
 // chunk of aux rows [P0, P0 + pc).
+// half (embedded tensors, n = 2 half): Y's rows (P, t) with all of t < half before those of t >= half, else in order.
 // A CTA takes a 32 x 32 tile (t, q) of a stretch of aux rows: the coefficients and gather offsets are read and formed once, each
 // B tile is transposed through shared memory.  Bound: B read twice, Y written once; with a thread per element four 64-bit
 // divisions, three coefficient reads and a column-wise read of B each: d = 240, naux = 480 270 us, now 139.
 template <int PL>
 __global__ void __launch_bounds__(256) hx_y_kernel(const double* B, int64_t P0, int64_t pc, int64_t n, const double* x2, const int64_t* pair_of,
-                                                   const double* l1, const double* l2, double* Y) {
+                                                   const double* l1, const double* l2, int64_t half, double* Y) {
   __shared__ double tile[PL][32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t nt = (n + 31) / 32, t0 = blockIdx.x / nt * 32, q0 = blockIdx.x % nt * 32, q = q0 + tx;
   double c[4], w[4] = {0.0, 0.0, 0.0, 0.0};
-  int64_t at[4] = {0, 0, 0, 0};
+  int64_t at[4] = {0, 0, 0, 0}, row0[4], rstep = half ? half : n;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int64_t t = t0 + ty + 8 * k;
     const bool in = t < n && q < n;
+    row0[k] = half && t >= half ? pc * half + (t - half) : t;
     c[k] = in ? -x2[q * n + t] : 0.0;
     if (in && pair_of) {
       const int64_t st = pair_of[t], qb = pair_of[q];
@@ -279,7 +281,7 @@ __global__ void __launch_bounds__(256) hx_y_kernel(const double* B, int64_t P0, 
         for (int z = 0; z < PL; ++z) {
           double v = c[k] * tile[z][tx][ty + 8 * k];
           if (pair_of) v += w[k] * g[k][z];
-          Y[((pl * n + t) * n + q) * PL + z] = v;
+          Y[((pl * rstep + row0[k]) * n + q) * PL + z] = v;
         }
       }
     }
@@ -551,7 +553,7 @@ void mo_jkl(rr_mo_store* m, const int64_t* pair_of, double* J, double* K, double
 // ---------------------------------------------------------------- generalized Fock
 
 // riHxFockGemm on a tensor Bt (naux, d*d) of element kind PL.  All matrix arguments on the device.
-void hx_fock_core(rr_mo_store* m, const double* Bt, int64_t d, int PL, const double* h, const double* occ,
+void hx_fock_core(rr_mo_store* m, const double* Bt, const double* Bs, int64_t d, int PL, const double* h, const double* occ,
                   const double* h2, const double* x2, const int64_t* pair_of, const double* l1, const double* l2,
                   double* F, cudaStream_t s) {
   const int64_t naux = m->naux;
@@ -582,7 +584,10 @@ void hx_fock_core(rr_mo_store* m, const double* Bt, int64_t d, int PL, const dou
   if (cplx) hx_f0f1_kernel<2><<<fgrid, 256, 0, s>>>(Bt, W, h, occ, naux, d, F);
   else hx_f0f1_kernel<1><<<fgrid, 256, 0, s>>>(Bt, W, h, occ, naux, d, F);
   RR_LAUNCH_CHECK();
-  // G = sum over aux chunks of B_view^T Y, B_view = (pc*d) x d rows (P,t), Y likewise
+  // G = sum over aux chunks of B_view^T Y, B_view = (pc*d) x d rows (P,t), Y likewise.  Of an embedded tensor (Bs: the spatial
+  // one) row (P, t) has only the columns of t's spin: two products with Bs over half the rows each, d = 240,
+  // naux = 480 548 us for the full one, now 324.
+  const int64_t half = Bs ? d / 2 : 0;
   const int64_t pc = chunk_rows(naux, PL * d * d);
   m->T.ensure(static_cast<size_t>(std::max<int64_t>(pc * PL * d * d, 1)));
   bool first = true;
@@ -590,8 +595,8 @@ void hx_fock_core(rr_mo_store* m, const double* Bt, int64_t d, int PL, const dou
     const int64_t cnt = std::min(pc, naux - P0);
     const int64_t tiles = ((d + 31) / 32) * ((d + 31) / 32);
     const dim3 ygrid(static_cast<unsigned>(tiles), static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(cnt, 2368 / tiles))));
-    if (cplx) hx_y_kernel<2><<<ygrid, 256, 0, s>>>(Bt, P0, cnt, d, x2, pair_of, l1, l2, m->T.p);
-    else hx_y_kernel<1><<<ygrid, 256, 0, s>>>(Bt, P0, cnt, d, x2, pair_of, l1, l2, m->T.p);
+    if (cplx) hx_y_kernel<2><<<ygrid, 256, 0, s>>>(Bt, P0, cnt, d, x2, pair_of, l1, l2, half, m->T.p);
+    else hx_y_kernel<1><<<ygrid, 256, 0, s>>>(Bt, P0, cnt, d, x2, pair_of, l1, l2, half, m->T.p);
     RR_LAUNCH_CHECK();
     GemmDesc g;
     g.cplx = cplx;
@@ -599,6 +604,13 @@ void hx_fock_core(rr_mo_store* m, const double* Bt, int64_t d, int PL, const dou
     g.A = Bt + PL * P0 * d * d; g.lda = d; g.opA = Op::T;
     g.B = m->T.p; g.ldb = d;
     g.C = G; g.ldc = d;
+    if (half) {
+      g.M = half; g.K = cnt * half;
+      g.A = Bs + P0 * half * half; g.lda = half;
+      g.batch = 2;
+      g.strideB = cnt * half * d;
+      g.strideC = half * d;
+    }
     g.beta = first ? 0.0 : 1.0;
     m->work.ensure(static_cast<size_t>(std::max<int64_t>(gemm_work_doubles(g), 1)));
     gemm(g, s, m->work.p, static_cast<int64_t>(m->work.n));
@@ -649,7 +661,7 @@ void mo_hx_fock(rr_mo_store* m, const double* h, const double* occ, const double
     }
     Bt = emb;
   }
-  hx_fock_core(m, Bt, d, PL, hd, od, h2d, x2d, pair_of ? pod : nullptr, l1d, l2d, Fd, s);
+  hx_fock_core(m, Bt, m->cplx ? nullptr : m->B.p, d, PL, hd, od, h2d, x2d, pair_of ? pod : nullptr, l1d, l2d, Fd, s);
   copy_out(F, Fd, PL * dd, host, s);
 }
 
