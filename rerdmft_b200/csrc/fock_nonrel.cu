@@ -433,17 +433,17 @@ void fock_nonrel(rr_ri_store* h, const double* hc, const double* D, const double
   }
   // J from the density on the side stream (after the upload of D there), beside the occupied
   // recovery (X^T (S D S / 2) X, eigenvalues > 0.5) as c_t = F^T X^T on s, then the exchange.
-  // One J CTA per SM: it shares the SMs with the recovery and then the half-transform (measured at
-  // n = 400, naux = 1600, nocc = 40: 1.67 ms per build with one, 1.70 with two, 1.81 with three);
-  // RR_J_CTAS=<k> sets another count for measurement.
-  static const int j_ctas = [] {
+  // The digit products of the exchange take whole SMs, so the J passes should be through when the recovery is: two CTAs per
+  // SM from 1e8 tensor elements on, one below, where they would only slow the recovery down.  One / two / three CTAs,
+  // us per build on device arrays: n = 160 283 / 283 / 292, n = 240 382 / 386 / 401, n = 320 (1.3e8) 586 / 578 / 591, n = 400 1129 /
+  // 1079 / 1085, n = 400 with 100 occupied 1980 / 1904 / 1954.  RR_J_CTAS=<k> sets another count for measurement.
+  static const int j_env = [] {
     const char* e = std::getenv("RR_J_CTAS");
-    const int k = e ? std::atoi(e) : 1;
-    return k >= 1 && k <= 4 ? k : 1;
+    const int k = e ? std::atoi(e) : 0;
+    return k >= 1 && k <= 4 ? k : 0;
   }();
-  // RR_J_AFTER_RECOVERY=1 (device pointers, for measurement): the J passes start after the recovery
-  // instead, beside the half-transform and the SYRK only: 1.630 / 1.748 / 1.818 ms per build with 1 / 2 / 3
-  // J CTAs per SM, against 1.565 / 1.584 / 1.708 ms from the top of the build.
+  const int j_ctas = j_env ? j_env : static_cast<double>(h->naux) * static_cast<double>(n2) >= 1e8 ? 2 : 1;
+  // RR_J_AFTER_RECOVERY=1 (device pointers, for measurement): the J passes start after the recovery instead.
   static const bool j_late = [] {
     const char* e = std::getenv("RR_J_AFTER_RECOVERY");
     return e && std::atoi(e) == 1;
