@@ -29,18 +29,10 @@ ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
 N_AO, N_AUX, N_OCC, SEED = 400, 1600, 40, 2024
-# The half-transform kernel of the nonrelativistic exchange (RR_HALF_TRANSFORM selects it; m16 is the
-# library default) with the DRAM bytes (read + write) of one launch at this workload from its ncu
-# capture (B read once, T written once), None where no capture exists.
-HT_KIND = os.environ.get("RR_HALF_TRANSFORM", "m16").split(":")[0]
-HT_KERNELS = {
-    "m8": dict(kernel="dgemm_kernel half-transform T^P = Ct B^P (FP64 DMMA m8n8k4)",
-               traffic=2.048888e9 + 0.194917e9, profile="profiles/dgemm_half_transform_n400_naux1600_nocc40.md"),
-    "m16": dict(kernel="ht_dmma16_kernel half-transform T^P = Ct B^P (FP64 DMMA m16n8k8)",
-                traffic=2.048169e9 + 0.197358e9,
-                profile="profiles/ht_dmma16_half_transform_n400_naux1600_nocc40.md"),
-}
-HT = HT_KERNELS[HT_KIND]
+# The half-transform kernel of the nonrelativistic exchange at this workload, and the bytes of one launch: the digit planes
+# of B (8 bytes an element, rows padded to 32) read once and those of T written once.
+HT_KERNEL = "oz_gemm_kernel half-transform T^P = Ct B^P (FP64 as INT8 digit planes, tcgen05 kind::i8)"
+HT_BYTES = 8.0 * N_AUX * (N_AO * (-(-N_AO // 32) * 32) + N_OCC * N_AO)
 METRIC = "RI J+K Fock builds/s"
 UNIT = "builds/s"
 
@@ -1176,16 +1168,14 @@ def main():
     hbm_peak, hbm_src = measured_peaks()
     fp64_peak = fp64_gemm_peak(torch) if rank == 0 else None
     ht_flops = 2.0 * N_AUX * N_OCC * N_AO * N_AO
-    # The exchange SYRK computes only the upper 80 x 80 output tiles of the symmetric K (15 of 25 at
-    # n = 400) and mirrors the rest: executed flops, not the full 2*naux*nocc*n^2 count.
-    syrk_tile = 80
-    syrk_nt = -(-N_AO // syrk_tile)
-    syrk_flops = 2.0 * N_AUX * N_OCC * (syrk_nt * (syrk_nt + 1) // 2) * syrk_tile * syrk_tile
+    # the SYRK's symmetric K: the products on and above the diagonal
+    syrk_flops = 1.0 * N_AUX * N_OCC * N_AO * (N_AO + 1)
     j_bytes = 2.0 * N_AUX * N_AO * N_AO * 8  # algorithmic: two passes over B
     # both passes stream the packed upper triangles of B (from the top of the build, beside the recovery)
     j_bytes_streamed = 2.0 * N_AUX * (-(-(N_AO * (N_AO + 1) // 2) // 32) * 32) * 8
     phases = {k: round(v, 4) for k, v in acc.items()}
     ht_tf = ht_flops / (acc["half_transform_ms"] / 1e3) / 1e12 if acc.get("half_transform_ms") else None
+    ht_gbs = HT_BYTES / (acc["half_transform_ms"] / 1e3) / 1e9 if acc.get("half_transform_ms") else None
     ex_tf = syrk_flops / (acc["exchange_ms"] / 1e3) / 1e12 if acc.get("exchange_ms") else None
     j_gbs = j_bytes_streamed / (acc["coulomb_ms"] / 1e3) / 1e9 if acc.get("coulomb_ms") else None
     k_ms = acc.get("half_transform_ms", 0.0) + acc.get("exchange_ms", 0.0)
@@ -1217,24 +1207,21 @@ def main():
         ms_per_step=1e3 * t / args.steps, higher_is_better=True, scaling="weak", vs_baseline=None, dtype="f64",
         data="synthetic",
         config=bench_config(ws),
-        roofline={"bound": "tensor", "kernel": HT["kernel"],
-                  "achieved": ht_tf, "peak": fp64_peak, "unit": "TFLOP/s",
-                  "frac": (ht_tf / fp64_peak) if (ht_tf and fp64_peak) else None, "traffic": HT["traffic"],
-                  "traffic_source": ("dram read+write of one launch, ncu capture in " + HT["profile"])
-                  if HT["traffic"] else "no ncu capture of this kernel yet",
-                  "algorithmic_bytes": 8.0 * N_AUX * (N_AO * N_AO + N_OCC * N_AO),
-                  "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (FP64 has no entry in MEASURED_PEAKS.json)",
-                  "algorithmic": "2*naux*nocc*n^2 flops per launch (one launch per build)"},
-        exchange={"bound": "tensor", "kernel": "half-transform + SYRK (FP64 DMMA)", "achieved": k_tf,
+        roofline={"bound": "hbm", "kernel": HT_KERNEL, "achieved": ht_gbs, "peak": hbm_peak, "unit": "GB/s",
+                  "frac": (ht_gbs / hbm_peak) if ht_gbs else None, "peak_source": hbm_src, "traffic": None,
+                  "traffic_source": "no ncu capture at this size (smaller ones: profiles/oz_gemm_digit_products.md)",
+                  "algorithmic_bytes": HT_BYTES, "fp64_tflops": ht_tf, "cublas_dgemm_tflops": fp64_peak,
+                  "algorithmic": "digit planes of B read once and of T written once (one launch per build)"},
+        exchange={"bound": "tensor", "kernel": "half-transform + SYRK (INT8 digit planes)", "achieved": k_tf,
                   "peak": fp64_peak, "unit": "TFLOP/s", "frac": (k_tf / fp64_peak) if (k_tf and fp64_peak) else None,
-                  "algorithmic": "2*naux*nocc*n^2 (half-transform) + 2*naux*nocc*15*80*80 (the SYRK's executed "
-                                 "upper tiles) flops per build"},
+                  "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (FP64 has no entry in MEASURED_PEAKS.json)",
+                  "algorithmic": "2*naux*nocc*n^2 (half-transform) + naux*nocc*n(n+1) (SYRK) FP64 flops per build"},
         coulomb={"bound": "hbm", "achieved": j_gbs, "peak": hbm_peak, "unit": "GB/s",
                  "frac": (j_gbs / hbm_peak) if j_gbs else None, "peak_source": hbm_src,
                  "algorithmic": "2*naux*n^2*8 bytes per build (two passes over B)",
                  "streamed": "2*naux*n(n+1)/2*8 bytes: both passes stream the packed upper triangles of the "
                              "symmetric B^P, on a side stream from the top of the build (beside the occupied "
-                             "recovery and the half-transform, one CTA per SM); achieved counts the streamed bytes",
+                             "recovery, two CTAs per SM); achieved counts the streamed bytes",
                  "algorithmic_rate_gbs": (j_bytes / (acc["coulomb_ms"] / 1e3) / 1e9) if acc.get("coulomb_ms") else None},
         kernels={"half_transform_tflops": ht_tf, "syrk_tflops_executed": ex_tf},
         phases_ms=phases, clocks=clk, e2e=e2e, gpu_launches=int(launches), cpu_baseline=cpu, parity=parity,
