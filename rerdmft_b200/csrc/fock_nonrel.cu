@@ -109,7 +109,7 @@ void exchange_nonrel(rr_ri_store* h, const double* Ct, int64_t ldct, bool ct_tra
     return;
   }
   if (K && !half_only && h->oz[0].ok && oz_worth(naux, n, nocc)) {
-    if (Dp) coulomb_early(h, Dp, Jout, s, 1);
+    if (Dp) coulomb_early(h, Dp, Jout, s, static_cast<double>(naux) * n * n >= 1e8 ? 2 : 1);  // (the rule of fock_nonrel)
     if (oz_exchange_nonrel(h, Ct, ldct, ct_transposed, nocc, K, s)) return;
     if (Dp) coulomb_join(h, s);  // no memory for the digit planes: the path below forms J again
   }

@@ -131,9 +131,10 @@ void launch_real(const Params& p, dim3 grid, cudaStream_t s) {
   launch_cfg<4, 4, 2, 2, AK, BKM, false>(p, grid, s);
 }
 
-// Complex products: 32 x 32 tiles with K split up to 4 ways up to n = 1024 (measured 97 instead of
-// 114 us for a Hermitian 800^3 product, 27 instead of 39 us at 400), 32 x 64 above.
-bool cplx_tile32(const GemmDesc& d) { return d.cplx && d.M <= 1024 && d.N <= 1024; }
+// Complex products: 32 x 32 tiles up to n = 2048, with K split up to 4 ways while that is below six rounds of tiles (measured 97
+// instead of 114 us for a Hermitian 800^3 product, 27 instead of 39 us at 400), 32 x 64 above.  32 x 64 / 32 x 32 without a
+// split, us: 1100^3 550 / 433, 1600 x 800 x 800 411 / 320, 1600 x 800 x 1600 791 / 620, 1600^3 1306 / 1144, 2000^3 2266 / 2229.
+bool cplx_tile32(const GemmDesc& d) { return d.cplx && d.M <= 2048 && d.N <= 2048; }
 
 Shape pick_shape(const GemmDesc& d) {
   if (cplx_tile32(d)) return {32, 32};
@@ -159,7 +160,7 @@ int pick_splits(const GemmDesc& d, Shape sh, int64_t* kchunk) {
   if (cplx_tile32(d) || (sh.bm == 32 && sh.bn == 32 && tiles < 2LL * num_sms())) {
     // small products (recovery, SCF): one wave of 32 x 32 tiles at most, so split K up to 4; up to 8, 16 where that
     // still leaves SMs idle
-    const int64_t most = 16 * tiles <= num_sms() ? 16 : 8 * tiles <= num_sms() ? 8 : 4;
+    const int64_t most = d.cplx && tiles >= 6 * num_sms() ? 1 : 16 * tiles <= num_sms() ? 16 : 8 * tiles <= num_sms() ? 8 : 4;
     splits = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(most, d.K / (4 * KT))));
   } else if (!(sh.bm == 32 && sh.bn == 32) && tiles < 2LL * num_sms() && d.K >= 8 * KT) {
     splits = static_cast<int>(std::min<int64_t>((target + tiles - 1) / tiles, d.K / (8 * KT)));
