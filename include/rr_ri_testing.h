@@ -83,6 +83,9 @@ int rr_test_chol_apply(const double* M, int64_t r, const double* Y, int64_t n, i
  * missed part of the spectrum or max_steps passed, 2 a grid barrier expired. */
 int rr_test_sp2(const double* F, int64_t n, double nocc, int32_t cplx, double lo, double hi, int32_t sure, int32_t max_steps,
                 double* X, double* outcome);
+/* Doubles of workspace the SCF loops reserve for the purification of an n x n problem, and the doubles its one launch
+ * addresses from the start of that workspace (0 where the step launches run).  No device work. */
+int rr_test_sp2_workspace(int64_t n, int32_t cplx, int64_t* reserved, int64_t* touched);
 /* [lo, hi] (host, in and out) narrowed to the widened extreme eigenvalues of T y = theta M y (32 x 32). */
 int rr_test_ritz(const double* T, const double* M, int32_t cplx, double* lo_hi);
 

@@ -174,6 +174,7 @@ _SIGS = {
                                           ctypes.POINTER(_vp), ctypes.POINTER(_i64), ctypes.POINTER(RankReport)]),
     "rr_test_chol_apply": (ctypes.c_int, [_vp, _i64, _vp, _i64, _i32, _i32, _vp, _vp, _vp]),
     "rr_test_sp2": (ctypes.c_int, [_vp, _i64, _d, _i32, _d, _d, _i32, _i32, _vp, _vp]),
+    "rr_test_sp2_workspace": (ctypes.c_int, [_i64, _i32, ctypes.POINTER(_i64), ctypes.POINTER(_i64)]),
     "rr_test_ritz": (ctypes.c_int, [_vp, _vp, _i32, _vp]),
     "rr_test_boys": (ctypes.c_int, [_vp, _i64, _i32, _vp]),
     "rr_ri_info": (ctypes.c_int, [_vp, ctypes.POINTER(_i64), ctypes.POINTER(_i64), ctypes.POINTER(_i64)]),

@@ -60,7 +60,7 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 
 // Two-stage reductions: RED_CTAS CTAs write one partial each (CTA b owns a fixed chunk), then one
 // CTA per row combines the partials in a fixed order, so sums are identical run to run.
-constexpr int RED_CTAS = 256;
+constexpr int RED_CTAS = kScfRedCtas;
 
 template <int OP>  // 0 sum, 1 min, 2 max
 __global__ void reduce_partials_kernel(const double* part, int cols, double scale, double* out) {
@@ -534,8 +534,7 @@ void ritz_bounds(rr_ri_store* h, const double* F, int64_t n, bool cplx, double* 
 // at most 120 steps.
 void sp2_projector(rr_ri_store* h, const double* F, int64_t n, int64_t nocc, double* Pi, double* T, double* scal,
                    cudaStream_t s, bool cplx) {
-  const int PL = cplx ? 2 : 1;
-  h->work.ensure(static_cast<size_t>(std::max<int64_t>(static_cast<int64_t>(h->work.n), 8 * n * n * PL + 6 * RED_CTAS)));
+  h->work.ensure(static_cast<size_t>(std::max<int64_t>(static_cast<int64_t>(h->work.n), sp2_workspace_doubles(n, cplx))));
   double* part = h->work.p;  // Gershgorin partials, then the SP2 trace partials
   const int gcta = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(RED_CTAS, (n + 7) / 8)));
   if (cplx) gershgorin_partial_kernel<2><<<gcta, 256, 0, s>>>(F, n, part);

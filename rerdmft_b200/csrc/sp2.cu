@@ -509,6 +509,10 @@ int tiles_of(int64_t n) {
 
 int64_t sp2_scratch_doubles() { return 4 * kMaxTiles + 32; }
 
+int64_t sp2_workspace_doubles(int64_t n, bool cplx) {
+  return std::max<int64_t>(8 * n * n * (cplx ? 2 : 1) + 6 * kScfRedCtas, sp2_scratch_doubles() + 4);
+}
+
 void sp2_run_group(const Sp2Problem* p, int count, const std::function<const void*(const void*, size_t)>& put, cudaStream_t s) {
   static std::atomic<bool> attr[kMaxDevices];
   once_per_device(attr, [] {

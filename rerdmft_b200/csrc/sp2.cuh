@@ -11,6 +11,9 @@ namespace rr {
 // 5.0, 240 9.2 / 7.1, 400 16.5 / 14.8; complex n = 232 4.0 / 3.3, 314 5.1 / 4.2.  Beyond that a step's products fill the GPU by themselves.
 constexpr int64_t kSp2MaxReal = 512, kSp2MaxComplex = 400;
 
+// CTAs of the SCF loops' two-stage reductions.
+constexpr int kScfRedCtas = 256;
+
 // Doubles of scratch sp2_run needs besides X's second buffer.
 int64_t sp2_scratch_doubles();
 
@@ -20,6 +23,10 @@ int64_t sp2_scratch_doubles();
 // tr X^2 of the last step; [3] = steps.
 void sp2_run(const double* F, int64_t n, double nocc, bool cplx, const double* b, bool sure, int max_steps, double* X,
              double* Y, double* scratch, double* outcome, cudaStream_t s);
+
+// Doubles sp2_projector (scf.cu) reserves for an n x n problem: its reductions and split-K sums, or the one launch's scratch and
+// outcome, whose size does not depend on n and is the larger of the two up to n = 8 (complex 6).
+int64_t sp2_workspace_doubles(int64_t n, bool cplx);
 
 // The same for complex problems side by side, each on its own group of CTAs with its own barrier (b holds the spectrum,
 // at most 120 steps).  put copies a table to the device for launches on s.

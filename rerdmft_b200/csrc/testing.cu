@@ -123,6 +123,13 @@ int rr_test_sp2(const double* F, int64_t n, double nocc, int32_t cplx, double lo
   }
 }
 
+int rr_test_sp2_workspace(int64_t n, int32_t cplx, int64_t* reserved, int64_t* touched) {
+  if (!reserved || !touched || n < 1) return RR_ERR_ARG;
+  *reserved = rr::sp2_workspace_doubles(n, cplx != 0);
+  *touched = n <= (cplx ? rr::kSp2MaxComplex : rr::kSp2MaxReal) ? rr::sp2_scratch_doubles() + 4 : 0;
+  return RR_OK;
+}
+
 int rr_test_ritz(const double* T, const double* M, int32_t cplx, double* lo_hi) {
   try {
     rr::set_last_error("");
