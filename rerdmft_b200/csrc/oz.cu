@@ -354,6 +354,13 @@ __device__ __forceinline__ unsigned square_sum(uint2 d) {
                                       __dp4a(static_cast<int>(d.y), static_cast<int>(d.y), 0)));
 }
 
+// Squares of the top 16 bits of eight values, from their two leading digit planes.
+__device__ __forceinline__ unsigned long long top_square_sum(uint2 a, uint2 b) {
+  const int ax = static_cast<int>(a.x), ay = static_cast<int>(a.y), bx = static_cast<int>(b.x), by = static_cast<int>(b.y);
+  const int aa = __dp4a(ax, ax, __dp4a(ay, ay, 0)), ab = __dp4a(ax, bx, __dp4a(ay, by, 0)), bb = __dp4a(bx, bx, __dp4a(by, by, 0));
+  return static_cast<unsigned long long>(aa * 65536ll + ab * 512ll + bb);
+}
+
 // Four lanes x four 64-bit values to their transpose: lane i gets the values that the quad's lanes hold at i.
 __device__ __forceinline__ void quad_transpose(uint64_t (&v)[4], int lane) {
   const bool b0 = lane & 1, b1 = lane & 2;
@@ -400,6 +407,7 @@ __device__ __forceinline__ void store_planes(const HalfArgs& g, const Item& t, c
   const double* sb = g.p.sb + t.n0;
   if constexpr (MODE == 0) {
     unsigned sq = 0;
+    unsigned long long mag = 0;
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int c = unit_col<0>(group, u);
@@ -414,9 +422,11 @@ __device__ __forceinline__ void store_planes(const HalfArgs& g, const Item& t, c
 #pragma unroll
         for (int p = 0; p < kDigits; ++p) *reinterpret_cast<uint2*>(dst + p * A_PLANE) = d[p];
         sq += square_sum(d[4]);
+        mag += top_square_sum(d[0], d[1]);
       }
     }
     if (sq) atomicAdd(o.sq[0] + r.a, static_cast<unsigned long long>(sq));
+    if (mag) atomicAdd(o.mag[0] + r.a, mag);
   } else if constexpr (MODE == 1) {
     const int c = t.n0 + unit_col<1>(group, 0), fcols = 2 * static_cast<int>(o.period);
     if (r.live && unit_col<1>(group, 0) < t.nt && c < 2 * fcols) {
@@ -426,6 +436,7 @@ __device__ __forceinline__ void store_planes(const HalfArgs& g, const Item& t, c
       double re[8], im[8], y[8];
       uint2 d[kDigits];
       unsigned sq = 0;
+      unsigned long long mag = 0;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const double2 s2 = __ldg(reinterpret_cast<const double2*>(sb + unit_col<1>(group, 0)) + i);
@@ -443,9 +454,13 @@ __device__ __forceinline__ void store_planes(const HalfArgs& g, const Item& t, c
         digits8(y, d);
 #pragma unroll
         for (int p = 0; p < kDigits; ++p) *reinterpret_cast<uint2*>(base + at + p * A_PLANE) = d[p];
-        if (v < 2) sq += square_sum(d[4]);
+        if (v < 2) {
+          sq += square_sum(d[4]);
+          mag += top_square_sum(d[0], d[1]);
+        }
       }
       if (sq) atomicAdd(o.sq[fl] + r.a, static_cast<unsigned long long>(sq));
+      if (mag) atomicAdd(o.mag[fl] + r.a, mag);
     }
   } else {
     // result row (Pl, c % per), K byte (c / per) chi + koff + a
@@ -780,8 +795,7 @@ __global__ void __launch_bounds__(256) digitize_columns_kernel(const double* B, 
 
 // Row scales of a half-transform's result, their exponents, the inverse scales its digits are cut with, and zeroes
 // for the digit squares.
-__global__ void row_scales_kernel(const double* cnorm, int64_t n, const double* norm, int64_t nnorm, int* e_out, double* scale,
-                                  double* tinv, unsigned long long* sq) {
+__global__ void row_scales_kernel(const double* cnorm, int64_t n, const double* norm, int64_t nnorm, const RowScales out) {
   __shared__ double red[32];
   double m = 0.0;
   for (int64_t i = threadIdx.x; i < nnorm; i += blockDim.x) m = nan_max(m, norm[i]);
@@ -794,11 +808,158 @@ __global__ void row_scales_kernel(const double* cnorm, int64_t n, const double* 
   for (int64_t a = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; a < padded;
        a += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int e = a < n ? exponent_of(cnorm[a] * m) : kExpZero;
-    scale[a] = scale_of(e, kRowShift);
+    out.scale[a] = scale_of(e, kRowShift);
     if (a >= n) continue;
-    e_out[a] = e;
-    tinv[a] = e >= kExpBad ? 0.0 : pow2i(31 - e);
-    sq[a] = 0;
+    out.e[a] = e;
+    out.tinv[a] = e >= kExpBad ? 0.0 : pow2i(31 - e);
+    out.sq[a] = 0;
+    out.rowmax[a] = 0.0;
+    out.mag[a] = e >= kExpBad || e <= kExpZero ? kMagNever : 0;
+  }
+}
+
+constexpr int kRefitWarps = 8, kRefitRows = 16;
+struct RefitFlavour {
+  const double *B, *c;  // coefficient (j, q): part p at c + j cj + q cq + p
+  int64_t pitch, cj, cq, tile_bytes;
+  int n;
+  uint8_t* pl[4];
+  RowScales row;
+};
+struct RefitArgs {
+  RefitFlavour f[4];
+  int nf, r;
+  int64_t naux, period;
+  double need;          // rows with mag below this
+};
+
+__device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
+}
+
+// PHASE 0: rowmax = the largest magnitude of every row concerned; 1: its digits at the exponent of that.  A CTA collects the rows
+// concerned of 256 at a time; a warp forms T of one aux row for 16 of them and 8 MT coefficient rows at a time on FP64 MMAs (tcgen05
+// has no FP64 kind), fragments straight from global memory: neighbouring rows share sectors of B, the coefficients lie in L2.
+// Bound: the launch where no row is concerned, the latency of the fragments for a few rows, the FP64 pipe for all of them.
+// J and K of n = 400, naux = 1600, 40 orbitals with 0 / 1 / 10 / 100 / 399 such rows: 1.01 / 1.15 / 1.16 / 1.98 / 4.45 ms; four
+// components nl = 200, ns = 600, naux = 1000, 40 spinors, 0 / 1 / 10 / 300 of a flavour: 8.1 / 8.6 / 8.7 / 18.3 ms.  Fock builds without
+// such rows: two launches more, 1129 -> 1133 us (n = 400), 1933 -> 1936 us (X2C nl = 200).
+template <int PHASE, int PARTS>
+__global__ void __launch_bounds__(32 * kRefitWarps, 2) refit_kernel(const __grid_constant__ RefitArgs g) {
+  constexpr int MT = PARTS == 1 ? 5 : 3, SETS = PARTS == 1 ? 1 : 4;
+  __shared__ int list[32 * kRefitWarps], total;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lr = lane >> 2, lc = lane & 3;
+  const int64_t warps = static_cast<int64_t>(gridDim.x) * kRefitWarps, me = static_cast<int64_t>(blockIdx.x) * kRefitWarps + warp;
+  int64_t seen = 0;  // items dealt out so far
+  for (int fi = 0; fi < g.nf; ++fi) {
+    const RefitFlavour& f = g.f[fi];
+    const int n = f.n;
+    for (int row0 = 0; row0 < n; row0 += 32 * kRefitWarps) {
+      const bool mine = row0 + tid < n && static_cast<double>(f.row.mag[row0 + tid]) < g.need;
+      if (!__syncthreads_or(mine)) continue;
+      if (tid == 0) total = 0;
+      __syncthreads();
+      for (int w = 0; w < kRefitWarps; ++w) {  // in the order of the rows
+        if (w == warp) {
+          const unsigned vote = __ballot_sync(0xffffffffu, mine);
+          if (mine) list[total + __popc(vote & ((1u << lane) - 1))] = row0 + tid;
+          __syncwarp();
+          if (lane == 0) total += __popc(vote);
+        }
+        __syncthreads();
+      }
+      const int count = total, groups = (count + kRefitRows - 1) / kRefitRows;
+      const int64_t items = static_cast<int64_t>(groups) * g.naux;
+      for (int64_t it = (me + warps - seen % warps) % warps; it < items; it += warps) {
+        const int gr = static_cast<int>(it / g.naux) * kRefitRows;
+        const int64_t P = it % g.naux;
+        if (P == 0 && lane < kRefitRows && gr + lane < count) {
+          const int a = list[gr + lane];
+          if (PHASE == 0) {
+            f.row.sq[a] = 0;
+          } else {
+            const int e = exponent_of(f.row.rowmax[a]);
+            f.row.e[a] = e;
+            f.row.scale[a] = scale_of(e, kRowShift);
+          }
+        }
+        const double *b0 = f.B + P * f.pitch + list[min(gr + lr, count - 1)], *b1 = f.B + P * f.pitch + list[min(gr + 8 + lr, count - 1)];
+        // this lane's results: rows (list) gr + 8 t + 2 lc + q, coefficient rows j0 + 8 m + lr
+        double mx[2][2] = {};
+        int e[2][2];
+        unsigned long long sq[2][2] = {};
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+            e[t][q] = PHASE ? exponent_of(f.row.rowmax[list[min(gr + 8 * t + 2 * lc + q, count - 1)]]) : 0;
+        for (int j0 = 0; j0 < g.r; j0 += 8 * MT) {
+          double acc[MT][PARTS][2][2] = {};
+          const double* cp[MT];
+#pragma unroll
+          for (int m = 0; m < MT; ++m) cp[m] = f.c + min(j0 + 8 * m + lr, g.r - 1) * f.cj;
+#pragma unroll 4
+          for (int q0 = 0; q0 < n; q0 += 4) {
+            const int64_t q = min(q0 + lc, n - 1);
+            const bool in = q0 + lc < n;
+            const double x0 = in ? b0[q * n] : 0.0, x1 = in ? b1[q * n] : 0.0;
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+              for (int p = 0; p < PARTS; ++p) {
+                const double v = cp[m][q * f.cq + p];
+                dmma_8x8x4(acc[m][p][0], v, x0);
+                dmma_8x8x4(acc[m][p][1], v, x1);
+              }
+          }
+#pragma unroll
+          for (int m = 0; m < MT; ++m) {
+            const int j = j0 + 8 * m + lr;
+            if (j >= g.r) continue;
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+#pragma unroll
+              for (int q = 0; q < 2; ++q) {
+                const double re = acc[m][0][t][q], im = acc[m][PARTS - 1][t][q];
+                if constexpr (PHASE == 0) {
+                  mx[t][q] = fmax(mx[t][q], fmax(fabs(re), fabs(im)));
+                } else {
+                  const int at = gr + 8 * t + 2 * lc + q;
+                  if (at >= count) continue;
+                  const double s32 = pow2i(31 - e[t][q]);
+                  const int64_t off = left_at(f.tile_bytes, list[at], static_cast<uint32_t>(P * g.period + j));
+#pragma unroll
+                  for (int v = 0; v < SETS; ++v) {
+                    if (!f.pl[v]) continue;
+                    const double y = v == 0 ? re : v == 1 ? im : 0.5 * (v == 2 ? re - im : re + im);
+                    const uint64_t d = digit_bytes(to_s64(y, s32));
+#pragma unroll
+                    for (int p = 0; p < kDigits; ++p) f.pl[v][off + p * A_PLANE] = static_cast<uint8_t>(d >> (8 * (7 - p)));
+                    const int d4 = static_cast<int8_t>(d >> 24);
+                    if (v < 2) sq[t][q] += static_cast<unsigned long long>(d4 * d4);
+                  }
+                }
+              }
+          }
+        }
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            for (int o = 4; o < 32; o <<= 1) {
+              if (PHASE == 0) mx[t][q] = fmax(mx[t][q], __shfl_xor_sync(0xffffffffu, mx[t][q], o));
+              else sq[t][q] += __shfl_xor_sync(0xffffffffu, sq[t][q], o);
+            }
+            const int at = gr + 8 * t + 2 * lc + q;
+            if (lr == 0 && at < count) {
+              if (PHASE == 0) atomic_max_nonneg(f.row.rowmax + list[at], mx[t][q]);
+              else atomicAdd(f.row.sq + list[at], sq[t][q]);
+            }
+          }
+      }
+      seen += items;
+      __syncthreads();  // the list is written again
+    }
   }
 }
 
@@ -869,7 +1030,41 @@ void digitize_range(const double* B, int64_t pitch, int64_t n, int64_t P0, int64
 }
 
 void row_scales(const double* cnorm, int64_t n, const double* norm, int64_t nnorm, const RowScales& out, cudaStream_t s) {
-  row_scales_kernel<<<grid1(n, 256), 256, 0, s>>>(cnorm, n, norm, nnorm, out.e, out.scale, out.tinv, out.sq);
+  row_scales_kernel<<<grid1(n, 256), 256, 0, s>>>(cnorm, n, norm, nnorm, out);
+  RR_LAUNCH_CHECK();
+}
+
+void refit_rows(const RefitRows* f, int nf, int64_t naux, int64_t r, int64_t period, cudaStream_t s) {
+  RR_REQUIRE(nf >= 1 && nf <= 4, RR_ERR_ARG, "oz: flavour count");
+  RefitArgs g{};
+  const bool pairs = f[0].c.kind == 2;
+  for (int i = 0; i < nf; ++i) {
+    RefitFlavour& d = g.f[i];
+    const CoefSrc& c = f[i].c;
+    RR_REQUIRE(c.kind <= 2 && (c.kind == 2) == pairs, RR_ERR_STATE, "oz: coefficient kinds");
+    d.B = f[i].B;
+    d.pitch = f[i].pitch;
+    d.c = c.kind == 2 ? c.src + 2 * c.off : c.src;
+    d.cj = c.kind == 0 ? c.ld : c.kind == 1 ? 1 : 2 * c.ld;
+    d.cq = c.kind == 0 ? 1 : c.kind == 1 ? c.ld : 2;
+    d.tile_bytes = Planes{nullptr, f[i].n, naux * period, kBM}.tile_bytes();
+    d.n = static_cast<int>(f[i].n);
+    for (int v = 0; v < 4; ++v) d.pl[v] = f[i].pl[v];
+    d.row = f[i].row;
+  }
+  g.nf = nf;
+  g.naux = naux;
+  g.r = static_cast<int>(r);
+  g.period = period;
+  g.need = 1073741824.0 / refit_limit(naux * period);  // mag is K_aa in units of 2^(2 e - 30)
+  const int grid = 2 * sm_count_current(), threads = 32 * kRefitWarps;
+  if (pairs) {
+    refit_kernel<0, 2><<<grid, threads, 0, s>>>(g);
+    refit_kernel<1, 2><<<grid, threads, 0, s>>>(g);
+  } else {
+    refit_kernel<0, 1><<<grid, threads, 0, s>>>(g);
+    refit_kernel<1, 1><<<grid, threads, 0, s>>>(g);
+  }
   RR_LAUNCH_CHECK();
 }
 

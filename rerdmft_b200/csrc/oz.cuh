@@ -16,6 +16,7 @@
 
 #include <cuda.h>
 
+#include <cmath>
 #include <cstdint>
 
 #include "rr_common.cuh"
@@ -93,11 +94,12 @@ void digitize_range(const double* B, int64_t pitch, int64_t n, int64_t P0, int64
 
 // Exponents of the half-transformed rows: e[a] for |sum_q B^P[q][a] c[q]|, every P and every coefficient row of norm
 // at most max(norm[0 .. nnorm)).  scale[a] = 2^(e - 35) (padded to a multiple of 64 entries), tinv[a] = 2^(31 - e),
-// sq[a] = 0.
+// sq[a] = 0, rowmax[a] = 0, mag[a] = 0 (kMagNever where e is no magnitude: a zero row or one that is not finite).
+constexpr unsigned long long kMagNever = 1ull << 62;
 struct RowScales {
   int* e = nullptr;
-  double *scale = nullptr, *tinv = nullptr;
-  unsigned long long* sq = nullptr;
+  double *scale = nullptr, *tinv = nullptr, *rowmax = nullptr;
+  unsigned long long *sq = nullptr, *mag = nullptr;
 };
 void row_scales(const double* cnorm, int64_t n, const double* norm, int64_t nnorm, const RowScales& out, cudaStream_t s);
 // The same for the MO transform: entry P per + j from pnorm[P] and the norm of coefficient column j (max over the ntab
@@ -110,12 +112,12 @@ struct HalfOut {
   int mode = 0;  // 0: real exchange planes, 1: complex exchange planes, 2: MO planes
   // mode 0 / 1: planes at row a, byte P period + j, inverse row scale tinv[a]; mode 1: two flavours of 2 period columns
   // (pair j, part) each, four plane sets Re, Im, (Re - Im) / 2, (Re + Im) / 2 (null: not wanted).  sq[a] +=
-  // the squares of digit 4 of the row (of Re and Im).
+  // the squares of digit 4 of the row (of Re and Im), mag[a] += the squares of its top 16 bits.
   int64_t period = 0;
   Planes t;                 // shape of every plane set
   uint8_t* pl[2][4] = {};
   const double* tinv[2] = {nullptr, nullptr};
-  unsigned long long* sq[2] = {nullptr, nullptr};
+  unsigned long long *sq[2] = {nullptr, nullptr}, *mag[2] = {nullptr, nullptr};
   // mode 2: row Pl per + c % per, byte (c / per) chi + koff + a with Pl = P - P0, inverse scale tinv[0][Pl per + c % per]
   int64_t per = 0, chi = 0, koff = 0;
   int64_t tile_bytes = 0;  // filled by half_product
@@ -124,6 +126,27 @@ struct HalfOut {
 // Aux rows P0 .. P0 + naux of the tensor; b: digit planes whose row 0 is aux row Pb (row (P - Pb) n + a).
 void half_product(const Planes& b, int64_t Pb, int64_t n, int64_t P0, int64_t naux, const double* cscale,
                   const Planes& coef, const double* coef_scale, int64_t ncol, const HalfOut& out, int* err, cudaStream_t s);
+
+// Rows of exchange planes whose exponent, a Cauchy-Schwarz bound, lies too far above their values: a product of two rows
+// a, b of kk terms drops about sqrt(7 kk) 74^2 2^-78 of 2^(ea + eb), which is measured against sqrt(K_aa K_bb), K_aa = sum T_a^2,
+// so its part grows with the square of rho = 2^e / sqrt(K_aa).  A row with rho^2 above refit_limit(kk) (that part above
+// 2^-50.5; kk = 64000 FP64 additions in a row leave about 2^-45) gets its true exponent: its T is formed again in FP64 and cut anew, and rho
+// is at most 2.01.  Such rows are rare (rho at the limits' sizes: at most 6.6 of 7.2 for n = 400, naux = 1600, 40 orbitals of the benchmark's
+// recipe, 7.9 of 8.1 for its four components; 3.5 of 13 for water and CO / cc-pVDZ at their SCF orbitals): nearly
+// dependent functions with large cancelling coefficients, functions far from every occupied orbital.
+inline double refit_limit(int64_t kk) {
+  const double r = 35118.0 / sqrt(7.0 * static_cast<double>(kk));
+  return r < 256.0 ? r : 256.0;
+}
+struct RefitRows {
+  const double* B = nullptr;  // the flavour's tensor, rows of n x n
+  int64_t pitch = 0, n = 0;
+  CoefSrc c;                  // its coefficients (kinds 0 - 2), as digitize_rows took them
+  uint8_t* pl[4] = {};        // its plane sets (HalfOut)
+  RowScales row;
+};
+// All flavours of a build (r coefficient rows or pairs, planes of shape (n, naux period)), after its half-transforms.
+void refit_rows(const RefitRows* f, int nf, int64_t naux, int64_t r, int64_t period, cudaStream_t s);
 
 // A list of products C_p[i][j] = sum_k A_p[i][k] B_p[j][k] of digit planes, one launch.
 struct Prod {

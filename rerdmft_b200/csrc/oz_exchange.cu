@@ -83,14 +83,16 @@ int64_t over_bytes(rr_ri_store* h, int t, int64_t n) {
 }
 
 // One allocation for the row scales of n rows.
-int64_t row_bytes(int64_t n) { return 8 * (round_up(n, 64) + 2 * round_up(n, 64)) + 4 * round_up(n, 64); }
+int64_t row_bytes(int64_t n) { return (8 * 5 + 4) * round_up(n, 64); }
 oz::RowScales rows_at(double* p, int64_t n) {
   const int64_t np = round_up(n, 64);
   oz::RowScales r;
   r.scale = p;
   r.tinv = p + np;
   r.sq = reinterpret_cast<unsigned long long*>(p + 2 * np);
-  r.e = reinterpret_cast<int*>(p + 3 * np);
+  r.mag = r.sq + np;
+  r.rowmax = p + 4 * np;
+  r.e = reinterpret_cast<int*>(p + 5 * np);
   return r;
 }
 
@@ -233,10 +235,17 @@ bool oz_exchange_nonrel(rr_ri_store* h, const double* Ct, int64_t ldct, bool ct_
   out.pl[0][0] = T.p;
   out.tinv[0] = row.tinv;
   out.sq[0] = row.sq;
+  out.mag[0] = row.mag;
   clear_tail(T, s);
   over_planes(h, 0, n, c.at<uint8_t>(o_b), s, [&](int64_t P0, int64_t cnt, const oz::Planes& b) {
     oz::half_product(b, P0, n, P0, cnt, h->oz[0].cscale, coef, cs, per, out, h->status.p, s);
   });
+  oz::RefitRows rf;
+  rf.B = h->B[0].p; rf.pitch = h->pitch[0]; rf.n = n;
+  rf.c = src;
+  rf.pl[0] = T.p;
+  rf.row = row;
+  oz::refit_rows(&rf, 1, naux, nocc, per, s);
   prof_mark(h, 2, s);
   pr.a = T; pr.b = T;
   pr.sa = row.scale; pr.sb = row.scale;
@@ -295,6 +304,7 @@ bool oz_exchange_rel(rr_ri_store* h, int nf, const int64_t* off, const int64_t* 
   }
   if (!c.commit()) return false;
   oz::RowScales row[4];
+  oz::RefitRows rf[4];
   for (int f = 0; f < nf; ++f) row[f] = rows_at(c.at<double>(o_row[f]), fs[f]);
 
   for (int g = 0; g < ng; ++g) {
@@ -314,6 +324,11 @@ bool oz_exchange_rel(rr_ri_store* h, int nf, const int64_t* off, const int64_t* 
       for (int v = 0; v < 4; ++v) out.pl[k][v] = o_t[f][v] >= 0 ? c.at<uint8_t>(o_t[f][v]) : nullptr;
       out.tinv[k] = row[f].tinv;
       out.sq[k] = row[f].sq;
+      out.mag[k] = row[f].mag;
+      rf[f].B = h->B[t].p; rf[f].pitch = h->pitch[t]; rf[f].n = n;
+      rf[f].c = src;
+      for (int v = 0; v < 4; ++v) rf[f].pl[v] = out.pl[k][v];
+      rf[f].row = row[f];
     }
     for (int k = 0; k < 2; ++k)
       oz::row_scales(h->oz[t].cnorm, n, norm + k * 2 * per, 2 * per, row[f0 + k], s);
@@ -323,8 +338,8 @@ bool oz_exchange_rel(rr_ri_store* h, int nf, const int64_t* off, const int64_t* 
     over_planes(h, t, n, c.at<uint8_t>(o_b[g]), s, [&](int64_t P0, int64_t cnt, const oz::Planes& b) {
       oz::half_product(b, P0, n, P0, cnt, h->oz[t].cscale, coef, cs, ncol, out, h->status.p, s);
     });
-
   }
+  oz::refit_rows(rf, nf, naux, r, per, s);
   prof_mark(h, 2, s);
 
   auto planes = [&](int f, int v) { return left(c.at<uint8_t>(o_t[f][v]), fs[f], kk); };
