@@ -1015,16 +1015,17 @@ void scf_x2c_grouped(rr_x2c_instance* ins, int64_t count, const rr_scf_opts* so,
     GLAUNCH(k_reduce<1>, 1, na, tab, al, P_GB, GRC, GRC, 1, 4, 1.0);
     GLAUNCH(k_reduce<2>, 1, na, tab, al, P_GB + GRC, GRC, GRC, 1, 5, 1.0);
     {
-      std::vector<int> sp = act;
-      int64_t widest = 0;
-      for (int i : act) widest = std::max(widest, b.gs[i].d.ne);
-      if (widest <= kSp2MaxComplex) {
-        // all steps of all instances in one launch (sp2.cu): 120 steps of a grouped product, a step launch and a host check
+      // Each instance by its own size (not by its neighbours': the two forms round differently, and an instance's result does
+      // not depend on the batch).  sp: what did not converge.
+      std::vector<int> one, sp, failed;
+      for (int i : act) (b.gs[i].d.ne <= kSp2MaxComplex ? one : sp).push_back(i);
+      if (!one.empty()) {
+        // all steps of all these in one launch (sp2.cu): 120 steps of a grouped product, a step launch and a host check
         // every fourth step took 4.7 ms of a scan of 12 instances of 40 - 144 spinors, this 1.4
         const int64_t per = sp2_scratch_doubles() + 4;
         b.c.sp2.ensure(static_cast<size_t>(per) * b.gs.size());
         std::vector<Sp2Problem> q;
-        for (int i : sp) {
+        for (int i : one) {
           const GDev& d = b.gs[i].d;
           double* w = b.c.sp2.p + per * i;
           q.push_back(Sp2Problem{d.Fo, d.scal + 4, d.Pi, d.T2, w, w + sp2_scratch_doubles(), static_cast<double>(d.r), d.ne});
@@ -1034,16 +1035,16 @@ void scf_x2c_grouped(rr_x2c_instance* ins, int64_t count, const rr_scf_opts* so,
         RR_CUDA(cudaMemcpy2DAsync(got.data(), 4 * sizeof(double), b.c.sp2.p + sp2_scratch_doubles(), per * sizeof(double),
                                   4 * sizeof(double), b.gs.size(), cudaMemcpyDeviceToHost, b.s));
         b.sync_scalars();
-        std::vector<int> keep;
-        for (int i : sp) {
+        tab = b.upload_tab();  // the read-back reset the table space
+        for (int i : one) {
           RR_REQUIRE(got[4 * i] != 2.0, RR_ERR_TIMEOUT, "rr_scf_run_x2c_grouped: a grid barrier of the density purification expired");
-          if (got[4 * i] != 0.0) keep.push_back(i);
+          if (got[4 * i] != 0.0) failed.push_back(i);
           sp2_max = std::max<int64_t>(sp2_max, static_cast<int64_t>(got[4 * i + 3]));
         }
-        sp.swap(keep);
-      } else {
-        GLAUNCH(k_sp2_init, GRC, na, tab, al);
-        const int* spl = al;
+      }
+      if (!sp.empty()) {
+        const int* spl = b.upload_list(sp);
+        GLAUNCH(k_sp2_init, GRC, sp.size(), tab, spl);
         // the same X^2 products every step: built once per stretch between read-backs, then re-launched
         GroupedPlan sq;
         bool sq_valid = false;
@@ -1083,6 +1084,7 @@ void scf_x2c_grouped(rr_x2c_instance* ins, int64_t count, const rr_scf_opts* so,
           }
         }
       }
+      sp.insert(sp.end(), failed.begin(), failed.end());
       for (int i : sp) {  // no gap at the Fermi level
         GHost& G = b.gs[i];
         G.in->status = RR_ERR_SOLVER;
