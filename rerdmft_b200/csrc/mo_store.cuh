@@ -10,6 +10,9 @@ struct rr_mo_store {
   rr::DevBuf<double> B;  // (naux, n*n) real, or complex interleaved
   // scratch
   rr::DevBuf<double> T, scratch, work, emb, hx, io;
+  // Digit planes and scales of an FP64 build of this tensor.  Here and not with the RI handle, which the builds only read: those of
+  // different tensors from one handle may run at the same time on different streams.
+  rr::DevBuf<uint8_t> ozbuf;
 };
 
 namespace rr {

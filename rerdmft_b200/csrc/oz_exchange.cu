@@ -449,7 +449,7 @@ bool mo_real(const double* B, int64_t pitch, int64_t n, int64_t naux, const doub
 bool oz_mo_build_nonrel(rr_ri_store* ri, const double* Cd, rr_mo_store* m, cudaStream_t s) {
   auto& z = ri->oz[0];
   if (!z.ok || !oz_worth(ri->naux, ri->n, ri->n)) return false;
-  Carve c(ri->ozbuf);
+  Carve c(m->ozbuf);
   return mo_real(ri->B[0].p, ri->pitch[0], ri->n, ri->naux, z.cscale, z.pnorm, z.planes, Cd, m->B.p, c, ri->status.p, s);
 }
 
@@ -463,7 +463,7 @@ bool oz_mo_build_ukb(rr_ri_store* ri, const double* cd, int64_t nt, rr_mo_store*
   for (int t = 0; t < 2; ++t)
     if (!ri->oz[t].planes) made += left_bytes(t ? ns : nl, t ? ns : nl);
   const int64_t pc = mo_range(naux, kDigits * nt * round_up(2 * nu, oz::kBK) + made);
-  Carve c(ri->ozbuf);
+  Carve c(m->ozbuf);
   int64_t o_coef[4], o_b[2];
   for (int f = 0; f < 4; ++f) o_coef[f] = c.take(coef_bytes(ncp, fs[f]));
   for (int t = 0; t < 2; ++t) {

@@ -29,7 +29,7 @@ struct rr_ri_store {
     double *cscale = nullptr, *cnorm = nullptr, *pnorm = nullptr;
     uint8_t* planes = nullptr;  // null: not kept
   } oz[2];
-  rr::DevBuf<uint8_t> ozbuf;  // digit planes, exponents and partial sums of one call
+  rr::DevBuf<uint8_t> ozbuf;  // digit planes, exponents and partial sums of one exchange
   // Scratch, grown on demand and reused across calls.
   rr::DevBuf<double> mats;  // per-call matrices (inputs, outputs, intermediates)
   rr::DevBuf<double> T;     // half-transformed exchange intermediate
