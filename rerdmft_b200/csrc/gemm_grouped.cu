@@ -429,7 +429,11 @@ struct Tuner {
 };
 
 Tuner& tuner() {
-  static Tuner* t = new Tuner();  // never destroyed: no CUDA calls during static destruction
+  static Tuner* t = [] {
+    auto* x = new Tuner();  // never destroyed: no CUDA calls during static destruction
+    x->ring.dev.library_own = x->cbuf.library_own = x->wbuf.library_own = true;
+    return x;
+  }();
   return *t;
 }
 

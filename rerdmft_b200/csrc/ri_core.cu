@@ -30,12 +30,13 @@ struct DevicePool {
   struct Live {
     size_t bytes;
     int dev;
+    bool own;
   };
   std::mutex mu;
   std::unordered_map<void*, Live> live;
   std::multimap<size_t, void*> kept[kMaxDevices];
   size_t kept_bytes[kMaxDevices] = {}, limit[kMaxDevices] = {};
-  int64_t live_count[kMaxDevices] = {};
+  int64_t live_count[kMaxDevices] = {};  // without the library's own
 
   void trim(int dev) {  // mu held
     for (auto& b : kept[dev]) cudaFree(b.second);
@@ -51,7 +52,7 @@ DevicePool& pool() {
 
 }  // namespace
 
-void* device_alloc(size_t bytes) {
+void* device_alloc(size_t bytes, bool own) {
   const int dev = current_device();
   const size_t unit = bytes >= (size_t{1} << 20) ? size_t{1} << 20 : 512, size = (bytes + unit - 1) / unit * unit;
   DevicePool& pl = pool();
@@ -62,10 +63,10 @@ void* device_alloc(size_t bytes) {
     auto it = pl.kept[dev].lower_bound(size);
     if (it != pl.kept[dev].end() && it->first <= size + size / 8) {
       p = it->second;
-      pl.live[p] = {it->first, dev};
+      pl.live[p] = {it->first, dev, own};
       pl.kept_bytes[dev] -= it->first;
       pl.kept[dev].erase(it);
-      ++pl.live_count[dev];
+      if (!own) ++pl.live_count[dev];
       return p;
     }
   }
@@ -81,15 +82,15 @@ void* device_alloc(size_t bytes) {
   if (e != cudaSuccess) throw Error(RR_ERR_CUDA, std::string("cudaMalloc failed: ") + cudaGetErrorString(e));
   if (pooled) {
     std::lock_guard<std::mutex> lock(pl.mu);
-    pl.live[p] = {size, dev};
-    ++pl.live_count[dev];
+    pl.live[p] = {size, dev, own};
+    if (!own) ++pl.live_count[dev];
   }
   return p;
 }
 
 void device_free(void* p) noexcept {
   DevicePool& pl = pool();
-  DevicePool::Live b{0, -1};
+  DevicePool::Live b{0, -1, false};
   {
     std::lock_guard<std::mutex> lock(pl.mu);
     auto it = pl.live.find(p);
@@ -113,7 +114,8 @@ void device_free(void* p) noexcept {
       size_t free_b = 0, total_b = 0;
       if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) pl.limit[b.dev] = total_b / kPoolShare;
     }
-    const bool last = --pl.live_count[b.dev] == 0;
+    if (!b.own) --pl.live_count[b.dev];
+    const bool last = pl.live_count[b.dev] == 0;
     if (ok && !last && pl.kept_bytes[b.dev] + b.bytes <= pl.limit[b.dev]) {
       pl.kept[b.dev].emplace(b.bytes, p);
       pl.kept_bytes[b.dev] += b.bytes;

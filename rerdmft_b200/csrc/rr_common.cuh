@@ -62,9 +62,9 @@ void count_device_alloc();
 // Device memory behind DevBuf (ri_core.cu).  device_free keeps a released block for a later device_alloc of about its
 // size on the same device, up to kPoolShare of the device's memory in all; a block that does not fit that
 // bound goes back to the driver at once, all of them do when the last DevBuf of the device is released or an allocation
-// fails.  Like cudaFree, device_free returns only after the work queued on the device is done, so a block never
+// fails.  Workspaces the library holds for the life of the process (own: DevBuf::library_own) don't count as that last one.  Like cudaFree, device_free returns only after the work queued on the device is done, so a block never
 // changes hands while a stream or a thread still uses it.
-void* device_alloc(size_t bytes);
+void* device_alloc(size_t bytes, bool own = false);
 void device_free(void* p) noexcept;
 
 // Owning device allocation, move-only.
@@ -72,6 +72,7 @@ template <typename T>
 struct DevBuf {
   T* p = nullptr;
   size_t n = 0;
+  bool library_own = false;  // set before the first allocation: not a user's object (device_alloc)
   DevBuf() = default;
   explicit DevBuf(size_t count) { alloc(count); }
   DevBuf(const DevBuf&) = delete;
@@ -85,7 +86,7 @@ struct DevBuf {
   void alloc(size_t count) {
     release();
     if (count) {
-      p = static_cast<T*>(device_alloc(count * sizeof(T)));
+      p = static_cast<T*>(device_alloc(count * sizeof(T), library_own));
       count_device_alloc();
     }
     n = count;

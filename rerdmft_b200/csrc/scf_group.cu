@@ -509,6 +509,7 @@ GroupCtx& group_ctx() {
     auto* c = new GroupCtx();  // kept for the process: its CUDA objects are never released at exit
     RR_CUDA(cudaStreamCreateWithFlags(&c->s, cudaStreamNonBlocking));
     for (auto& e : c->ev) RR_CUDA(cudaEventCreate(&e));
+    c->ring.dev.library_own = c->work.library_own = c->scal_all.library_own = c->sp2.library_own = c->status_all.library_own = true;
     c->ring.reserve(size_t{8} << 20);
     ctx[d] = c;
   }
