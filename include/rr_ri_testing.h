@@ -68,8 +68,8 @@ int rr_test_half_transform(const double* Ct, int64_t nocc, const double* B, int6
 int rr_test_half_transform_time(const double* Ct, int64_t nocc, const double* B, int64_t naux, int64_t n, double* T,
                                 int32_t variant, int32_t reps, double* ms);
 
-/* Releases the resident digit planes of a store (rr_ri_create*), as if they had not fitted: its FP64 products then
- * digitize ranges of aux rows on the fly.  *had = 1 when there were any. */
+/* Releases the digit planes of a store (rr_ri_create*; made first where no product has yet), as if they had not fitted: its FP64
+ * products then digitize ranges of aux rows on the fly.  *had = 1 when there were any. */
 int rr_test_drop_digit_planes(void* ri_handle, int32_t* had);
 
 /* out = Y L^-dagger (times_l 0) or Y L (1) for M = L L^dagger (r x r) and n rows of Y (row-major, interleaved when cplx) by the

@@ -8,7 +8,6 @@
 
 #include "grouped.cuh"
 #include "mo_store.cuh"
-#include "oz_paths.cuh"
 
 namespace rr {
 extern thread_local std::string g_last_error;
@@ -150,7 +149,6 @@ int rr_ri_create(const double* B, int64_t naux, int64_t n, int32_t mem, rr_ri_ha
       RR_CUDA(cudaMemsetAsync(h->status.p, 0, 2 * sizeof(int), h->ctx.main));
       upload_tensor(h->B[0], &h->pitch[0], B, naux, n * n, mem == RR_MEM_HOST, h->ctx.main);
       rr::pack_for_j(h, 0, n, h->ctx.main);
-      rr::oz_prepare(h, 0, n, h->ctx.main);
       RR_CUDA(cudaStreamSynchronize(h->ctx.main));
     } catch (...) {
       h->ctx.destroy();
@@ -182,8 +180,6 @@ int rr_ri_create_4c(const double* B_LL, const double* B_SS, int64_t naux, int64_
       upload_tensor(h->B[1], &h->pitch[1], B_SS, naux, ns * ns, mem == RR_MEM_HOST, h->ctx.main);
       rr::pack_for_j(h, 0, nl, h->ctx.main);
       rr::pack_for_j(h, 1, ns, h->ctx.main);
-      rr::oz_prepare(h, 0, nl, h->ctx.main);
-      rr::oz_prepare(h, 1, ns, h->ctx.main);
       RR_CUDA(cudaStreamSynchronize(h->ctx.main));
     } catch (...) {
       h->ctx.destroy();

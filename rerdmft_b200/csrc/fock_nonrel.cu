@@ -108,10 +108,13 @@ void exchange_nonrel(rr_ri_store* h, const double* Ct, int64_t ldct, bool ct_tra
     if (Dp) coulomb_after_ht(h, Dp, Ct, 0, Jout, nullptr, 0, s);
     return;
   }
-  if (K && !half_only && h->oz[0].ok && oz_worth(naux, n, nocc)) {
-    if (Dp) coulomb_early(h, Dp, Jout, s, static_cast<double>(naux) * n * n >= 1e8 ? 2 : 1);  // (the rule of fock_nonrel)
-    if (oz_exchange_nonrel(h, Ct, ldct, ct_transposed, nocc, K, s)) return;
-    if (Dp) coulomb_join(h, s);  // no memory for the digit planes: the path below forms J again
+  if (K && !half_only && oz_worth(naux, n, nocc)) {
+    const OzUse use(h, s);
+    if (use.ok) {
+      if (Dp) coulomb_early(h, Dp, Jout, s, static_cast<double>(naux) * n * n >= 1e8 ? 2 : 1);  // (the rule of fock_nonrel)
+      if (oz_exchange_nonrel(h, Ct, ldct, ct_transposed, nocc, K, s)) return;
+      if (Dp) coulomb_join(h, s);  // no memory for the digit planes: the path below forms J again
+    }
   }
   h->T.ensure(static_cast<size_t>(naux * nocc * n));
   GemmDesc ht;

@@ -130,12 +130,12 @@ void half_product(const Planes& b, int64_t Pb, int64_t n, int64_t P0, int64_t na
 // Rows of exchange planes whose exponent, a Cauchy-Schwarz bound, lies too far above their values: a product of two rows
 // a, b of kk terms drops about sqrt(7 kk) 74^2 2^-78 of 2^(ea + eb), which is measured against sqrt(K_aa K_bb), K_aa = sum T_a^2,
 // so its part grows with the square of rho = 2^e / sqrt(K_aa).  A row with rho^2 above refit_limit(kk) (that part above
-// 2^-50.5; kk = 64000 FP64 additions in a row leave about 2^-45) gets its true exponent: its T is formed again in FP64 and cut anew, and rho
-// is at most 2.01.  Such rows are rare (rho at the limits' sizes: at most 6.6 of 7.2 for n = 400, naux = 1600, 40 orbitals of the benchmark's
-// recipe, 7.9 of 8.1 for its four components; 3.5 of 13 for water and CO / cc-pVDZ at their SCF orbitals): nearly
+// 2^-50; kk = 64000 FP64 additions in a row leave about 2^-45) gets its true exponent: its T is formed again in FP64 and cut anew, and rho
+// is at most 2.01.  Such rows are rare (rho at the limits' sizes: at most 6.6 of 8.6 for n = 400, naux = 1600, 40 orbitals of the benchmark's
+// recipe, 7.9 of 9.7 for its four components; 3.5 of 13 for water and CO / cc-pVDZ at their SCF orbitals): nearly
 // dependent functions with large cancelling coefficients, functions far from every occupied orbital.
 inline double refit_limit(int64_t kk) {
-  const double r = 35118.0 / sqrt(7.0 * static_cast<double>(kk));
+  const double r = 49664.0 / sqrt(7.0 * static_cast<double>(kk));
   return r < 256.0 ? r : 256.0;
 }
 struct RefitRows {

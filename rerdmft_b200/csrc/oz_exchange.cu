@@ -171,46 +171,104 @@ __global__ void place_blocks_kernel(const __grid_constant__ BlockList l, double*
 
 }  // namespace
 
+namespace {
+
+// Column statistics and digit planes of tensor t (n x n rows); synchronises s.
 void oz_prepare(rr_ri_store* h, int t, int64_t n, cudaStream_t s) {
   auto& z = h->oz[t];
-  z.ok = false;
-  z.planes = nullptr;
-  z.buf.release();
-  if (h->naux == 0 || n < kOzMinDim || n > oz::kOzMaxK || h->naux * n >= (1LL << 31)) return;
-  // One allocation: a store's creation waits for each.
-  Carve c(z.buf);
+  if (h->naux == 0 || n < kOzMinDim || n > oz::kOzMaxK || h->naux * n >= (1LL << 31)) {
+    z.made = true;
+    return;
+  }
+  Carve c(z.stats);
   const int64_t o_cs = c.take(8 * h->naux * n), o_cn = c.take(8 * n), o_pn = c.take(8 * h->naux), o_flag = c.take(4);
-  const int64_t small = c.used, bytes = left_bytes(h->naux * n, n);
+  if (!c.commit()) return;  // no room now
   size_t free_b = 0, total_b = 0;
   RR_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  const int64_t o_pl = c.take(bytes);
-  bool keep = static_cast<double>(bytes) <= 0.25 * static_cast<double>(free_b) && c.commit();
-  if (!keep) {  // the products digitize ranges
-    c.used = small;
-    if (!c.commit()) return;
-  }
+  const int64_t bytes = left_bytes(h->naux * n, n);
+  Carve cp(z.buf);
+  cp.take(bytes);
+  const bool keep = static_cast<double>(bytes) <= 0.25 * static_cast<double>(free_b) && cp.commit();  // else: ranges
   z.cscale = c.at<double>(o_cs);
   z.cnorm = c.at<double>(o_cn);
   z.pnorm = c.at<double>(o_pn);
   int* flag = c.at<int>(o_flag);
-  if (keep) z.planes = c.at<uint8_t>(o_pl);
-  const oz::Planes pl = left(z.planes, h->naux * n, n);
+  const oz::Planes pl = left(keep ? z.buf.p : nullptr, h->naux * n, n);
   oz::digitize_columns(h->B[t].p, h->pitch[t], n, h->naux, keep ? &pl : nullptr,
                        oz::ColumnStats{z.cscale, z.cnorm, z.pnorm, flag}, s);
   int bad = 0;
   RR_CUDA(cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, s));
   RR_CUDA(cudaStreamSynchronize(s));
   z.ok = bad == 0;
-  if (!z.ok) {
-    z.planes = nullptr;
+  z.made = true;
+  if (z.ok) {
+    z.planes = keep ? z.buf.p : nullptr;
+  } else {
+    z.stats.release();
     z.buf.release();
   }
+}
+
+// Every store, for release_idle_planes.
+struct StoreList {
+  std::mutex mu;
+  std::vector<rr_ri_store*> all;
+};
+StoreList& stores() {
+  static StoreList* l = new StoreList();  // never destroyed: handles may outlive static destructors
+  return *l;
+}
+
+}  // namespace
+
+bool release_idle_planes(int device) noexcept {
+  bool any = false;
+  StoreList& l = stores();
+  std::lock_guard<std::mutex> lock(l.mu);
+  for (rr_ri_store* h : l.all) {
+    std::lock_guard<std::mutex> own(h->oz_mu);
+    if (h->oz_users > 0 || h->oz_pinned || h->ctx.device != device) continue;
+    for (auto& z : h->oz)
+      if (z.planes) {
+        z.planes = nullptr;
+        z.buf.release();  // (waits for the products queued on it)
+        any = true;
+      }
+  }
+  return any;
+}
+
+OzUse::OzUse(rr_ri_store* h, cudaStream_t s) : h_(h) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  RR_CUDA(cudaStreamIsCapturing(s, &capture));
+  const bool captured = capture != cudaStreamCaptureStatusNone;
+  {
+    std::lock_guard<std::mutex> lock(h->oz_mu);
+    ++h->oz_users;
+    if (captured) h->oz_pinned = true;
+  }
+  try {
+    std::lock_guard<std::mutex> lock(h->oz_making);
+    ok = true;
+    for (int t = 0; t < h->ntens; ++t) {
+      if (!h->oz[t].made && !captured) oz_prepare(h, t, t ? h->ns : h->n, s);
+      ok = ok && h->oz[t].ok;
+    }
+  } catch (...) {
+    std::lock_guard<std::mutex> lock(h->oz_mu);
+    --h->oz_users;
+    throw;
+  }
+}
+
+OzUse::~OzUse() {
+  std::lock_guard<std::mutex> lock(h_->oz_mu);
+  --h_->oz_users;
 }
 
 bool oz_exchange_nonrel(rr_ri_store* h, const double* Ct, int64_t ldct, bool ct_transposed, int64_t nocc, double* K,
                         cudaStream_t s) {
   const int64_t n = h->n, naux = h->naux;
-  if (!h->oz[0].ok || !oz_worth(naux, n, nocc)) return false;
   const int64_t per = round_up(nocc, 8), ncp = round_up(per, 16), kk = naux * per, ldo = round_up(n, 4);
   if (kk >= (1LL << 31)) return false;
   oz::Prod pr;
@@ -263,11 +321,11 @@ bool oz_exchange_rel(rr_ri_store* h, int nf, const int64_t* off, const int64_t* 
   const int64_t naux = h->naux;
   const int64_t per = round_up(std::max<int64_t>(r, 1), 8), kk = naux * per;
   if (r == 0 || kk >= (1LL << 31) || nf < 2 || nf > 4) return false;
-  for (int f = 0; f < nf; ++f)
-    if (!h->oz[tens[f]].ok) return false;
   // two flavours per tensor, side by side
   for (int f = 0; f < nf; f += 2)
     if (f + 1 >= nf || tens[f] != tens[f + 1] || fs[f] != fs[f + 1]) return false;
+  const OzUse use(h, s);
+  if (!use.ok) return false;
   const int ng = nf / 2;
   const int64_t ncol = 4 * per, ncp = round_up(ncol, 32);
 
@@ -447,8 +505,10 @@ bool mo_real(const double* B, int64_t pitch, int64_t n, int64_t naux, const doub
 }  // namespace
 
 bool oz_mo_build_nonrel(rr_ri_store* ri, const double* Cd, rr_mo_store* m, cudaStream_t s) {
+  if (!oz_worth(ri->naux, ri->n, ri->n)) return false;
+  const OzUse use(ri, s);
+  if (!use.ok) return false;
   auto& z = ri->oz[0];
-  if (!z.ok || !oz_worth(ri->naux, ri->n, ri->n)) return false;
   Carve c(m->ozbuf);
   return mo_real(ri->B[0].p, ri->pitch[0], ri->n, ri->naux, z.cscale, z.pnorm, z.planes, Cd, m->B.p, c, ri->status.p, s);
 }
@@ -457,7 +517,9 @@ bool oz_mo_build_ukb(rr_ri_store* ri, const double* cd, int64_t nt, rr_mo_store*
   const int64_t nl = ri->n, ns = ri->ns, naux = ri->naux, nu = 2 * nl + 2 * ns;
   const int64_t off[4] = {0, nl, 2 * nl, 2 * nl + ns}, fs[4] = {nl, nl, ns, ns};
   const int tens[4] = {0, 0, 1, 1};
-  if (!ri->oz[0].ok || !ri->oz[1].ok || 2 * nu > oz::kOzMaxK || nt == 0 || naux == 0) return false;
+  if (2 * nu > oz::kOzMaxK || nt == 0 || naux == 0) return false;
+  const OzUse use(ri, s);
+  if (!use.ok) return false;
   const int64_t nc = 2 * nt, ncp = round_up(nc, 16);
   int64_t made = 0;
   for (int t = 0; t < 2; ++t)
@@ -523,3 +585,15 @@ bool oz_mo_build_ukb(rr_ri_store* ri, const double* cd, int64_t nt, rr_mo_store*
 }
 
 }  // namespace rr
+
+rr_ri_store::rr_ri_store() {
+  auto& l = rr::stores();
+  std::lock_guard<std::mutex> lock(l.mu);
+  l.all.push_back(this);
+}
+
+rr_ri_store::~rr_ri_store() {
+  auto& l = rr::stores();
+  std::lock_guard<std::mutex> lock(l.mu);
+  l.all.erase(std::find(l.all.begin(), l.all.end(), this));
+}

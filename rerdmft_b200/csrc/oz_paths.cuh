@@ -19,10 +19,22 @@ inline bool oz_worth(int64_t naux, int64_t n, int64_t cols) {
   return n >= kOzMinDim && static_cast<double>(naux) * static_cast<double>(n) * static_cast<double>(n) * static_cast<double>(cols) >= 2e8;
 }
 
-// Column statistics and digit planes of tensor t (n x n rows); called when the store is filled, synchronises s.
-void oz_prepare(rr_ri_store* h, int t, int64_t n, cudaStream_t s);
+// The digit data of a store for the time in which a call queues products on it: made on the first use (statistics and planes of
+// every tensor; synchronises s), and held against release_idle_planes.  ok: the store's tensors are for the digit path.  Not
+// made while s is captured (the call then takes the DMMA path).
+class OzUse {
+ public:
+  OzUse(rr_ri_store* h, cudaStream_t s);
+  ~OzUse();
+  OzUse(const OzUse&) = delete;
+  OzUse& operator=(const OzUse&) = delete;
+  bool ok = false;
 
-// K = sum_P (Ct B^P)^T (Ct B^P); Ct as for exchange_nonrel.
+ private:
+  rr_ri_store* h_;
+};
+
+// K = sum_P (Ct B^P)^T (Ct B^P); Ct as for exchange_nonrel.  The caller holds an OzUse that is ok.
 bool oz_exchange_nonrel(rr_ri_store* h, const double* Ct, int64_t ldct, bool ct_transposed, int64_t nocc, double* K,
                         cudaStream_t s);
 

@@ -78,6 +78,17 @@ void* device_alloc(size_t bytes, bool own) {
       pl.trim(dev);
     }
     e = cudaMalloc(&p, size);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      // digit planes are copies that no call needs: stores that are not queueing products give theirs back
+      if (release_idle_planes(dev)) {
+        {
+          std::lock_guard<std::mutex> lock(pl.mu);
+          pl.trim(dev);
+        }
+        e = cudaMalloc(&p, size);
+      }
+    }
   }
   if (e != cudaSuccess) throw Error(RR_ERR_CUDA, std::string("cudaMalloc failed: ") + cudaGetErrorString(e));
   if (pooled) {

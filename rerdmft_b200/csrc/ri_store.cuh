@@ -2,6 +2,7 @@
 #pragma once
 
 #include <functional>
+#include <mutex>
 
 #include "gemm_f64.cuh"
 #include "j_stream.cuh"
@@ -9,6 +10,8 @@
 #include "rr_common.cuh"
 
 struct rr_ri_store {
+  rr_ri_store();   // in the list that release_idle_planes walks
+  ~rr_ri_store();
   rr::Context ctx;
   int64_t naux = 0, n = 0, ns = 0;  // n = nl for the 4c store
   int ntens = 1;
@@ -19,16 +22,19 @@ struct rr_ri_store {
   rr::DevBuf<double> Bpk[2];
   int64_t pitch_pk[2] = {0, 0};
   rr::DevBuf<int> status;   // device status word written by bounded waits
-  // Column scales, norms and digit planes of B[t] for the INT8 products (oz.cuh), filled with the store.  ok is
-  // false when B holds a NaN, an infinity or a value beyond 1e140, or n is too small for that path.  The
-  // planes (as large as B) are kept when they fit in a quarter of the free memory; otherwise the products
-  // digitize ranges of aux rows into their scratch.
+  // Column scales, norms and digit planes of B[t] for the INT8 products (oz.cuh), made by the first product that takes them
+  // (oz_paths.cuh): stores of small systems, Coulomb or mixed builds alone and the lockstep scans never carry them.  The
+  // planes (as large as B) are kept when they fit in a quarter of the free memory; otherwise, and after they were
+  // given back to a failing allocation, the products digitize ranges of aux rows into their scratch.
   struct {
-    bool ok = false;
-    rr::DevBuf<uint8_t> buf;  // all of the below
+    bool made = false, ok = false;  // ok: B holds no NaN, infinity or value beyond 1e140, and n is large enough
+    rr::DevBuf<uint8_t> stats, buf;
     double *cscale = nullptr, *cnorm = nullptr, *pnorm = nullptr;
     uint8_t* planes = nullptr;  // null: not kept
   } oz[2];
+  std::mutex oz_making, oz_mu;  // oz_mu: the two below, and planes that are given back
+  int oz_users = 0;             // calls that are queueing products on the planes
+  bool oz_pinned = false;       // a captured graph reads the planes: they stay
   rr::DevBuf<uint8_t> ozbuf;  // digit planes, exponents and partial sums of one exchange
   // Scratch, grown on demand and reused across calls.
   rr::DevBuf<double> mats;  // per-call matrices (inputs, outputs, intermediates)

@@ -66,6 +66,9 @@ void count_device_alloc();
 // changes hands while a stream or a thread still uses it.
 void* device_alloc(size_t bytes, bool own = false);
 void device_free(void* p) noexcept;
+// Gives the digit planes of the device's stores back (oz_exchange.cu), except where a call is queueing products on them or a captured
+// graph reads them; false: there were none.
+bool release_idle_planes(int device) noexcept;
 
 // Owning device allocation, move-only.
 template <typename T>

@@ -14,7 +14,6 @@
 #include <vector>
 
 #include "ri_store.cuh"
-#include "oz_paths.cuh"
 
 namespace rr {
 
@@ -344,7 +343,6 @@ int rr_ri_create_raw(const double* raw, int64_t naux_raw, int64_t n_ao, const do
         RR_CUDA(cudaStreamSynchronize(s));
       }
       rr::pack_for_j(h, 0, n_out, s);
-      rr::oz_prepare(h, 0, n_out, s);
       RR_CUDA(cudaStreamSynchronize(s));
     } catch (...) {
       h->ctx.destroy();

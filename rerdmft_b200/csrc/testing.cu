@@ -3,6 +3,7 @@
 #include <algorithm>
 
 #include "chol.cuh"
+#include "oz_paths.cuh"
 #include "ri_store.cuh"
 #include "sp2.cuh"
 #include "gemm_f64.cuh"
@@ -77,6 +78,7 @@ int rr_test_drop_digit_planes(void* ri_handle, int32_t* had) {
     rr::set_last_error("");
     auto* h = static_cast<rr_ri_store*>(ri_handle);
     RR_REQUIRE(h && had, RR_ERR_ARG, "rr_test_drop_digit_planes: null argument");
+    { const rr::OzUse use(h, h->ctx.main); }  // makes them, if no product has yet
     RR_CUDA(cudaDeviceSynchronize());
     *had = 0;
     for (auto& z : h->oz) {
