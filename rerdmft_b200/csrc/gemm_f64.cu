@@ -160,7 +160,11 @@ int pick_splits(const GemmDesc& d, Shape sh, int64_t* kchunk) {
   if (cplx_tile32(d) || (sh.bm == 32 && sh.bn == 32 && tiles < 2LL * num_sms())) {
     // small products (recovery, SCF): one wave of 32 x 32 tiles at most, so split K up to 4; up to 8, 16 where that
     // still leaves SMs idle
-    const int64_t most = d.cplx && tiles >= 6 * num_sms() ? 1 : 16 * tiles <= num_sms() ? 16 : 8 * tiles <= num_sms() ? 8 : 4;
+    // Flat complex products beyond 1024 (coefficient rows of a four-component recovery, up to 32 of them; half the SMs or fewer have a tile): K
+    // up to 8 ways, 32 x 64 tiles in up to 12 ranges / 4 / 8, us: 8 x 1100^2 21 / 22 / 18.5, 8 x 1600^2 31 / 41 / 33, 32 x 1600^2 35 / 46 / 35,
+    // 24 x 2000^2 59 / 57 / 51, 1600 x 32 x 1600 58 / 46 / 35; from 33 rows on 4 ways are as good (40 x 1600^2 60 / 60).
+    const bool flat = d.cplx && 2 * tiles <= num_sms() && std::max(d.M, d.N) > 1024;
+    const int64_t most = d.cplx && tiles >= 6 * num_sms() ? 1 : 16 * tiles <= num_sms() ? 16 : flat || 8 * tiles <= num_sms() ? 8 : 4;
     splits = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(most, d.K / (4 * KT))));
   } else if (!(sh.bm == 32 && sh.bn == 32) && tiles < 2LL * num_sms() && d.K >= 8 * KT) {
     splits = static_cast<int>(std::min<int64_t>((target + tiles - 1) / tiles, d.K / (8 * KT)));
