@@ -2,9 +2,9 @@
 //
 // Schedule for one call (stream `s` plus the handle's side stream):
 //   side: J pass 1 (gamma = B vec D) -> J pass 2 (J = B^T gamma) -> J finish     [HBM-bound]
-//   main: occupied recovery (S D S, X^T (.) X / 2, dsyevd, C_occ^T = Y_occ^T X^T)
-//         half-transform T[P] = C_occ^T B^P (batched DMMA GEMM)                  [FP64 tensor]
-//         K' = sum_P T[P]^T T[P] (split-K DMMA SYRK, upper tiles + mirror)        [FP64 tensor]
+//   main: occupied recovery (P_eff = X^T S D S X / 2, sign iteration, CholeskyQR; recovery.cu)   [latency]
+//         half-transform T[P] = C_occ^T B^P and K' = sum_P T[P]^T T[P] (split K, upper tiles) on INT8 digit planes (oz.cu)
+//         [tensor pipe, shared memory], or on FP64 DMMA where those are not worth it or not to be had
 //   join, F = h + J - K'   (K' = K/2 of the reference: its c_t carries sqrt(2)).
 #include <algorithm>
 #include <vector>
@@ -41,59 +41,6 @@ void coulomb_run(rr_ri_store* h, const double* tgam, int tseg, cudaStream_t s);
 void coulomb_join(rr_ri_store* h, cudaStream_t s);
 void coulomb_early(rr_ri_store* h, const double* Dp, double* J, cudaStream_t s, int ctas_per_sm);
 
-namespace {
-
-// K = sum_c parts[c] in the order c = 0, 1, ... (n2 entries each).
-__global__ void sum_parts_kernel(double* K, const double* parts, int nparts, int64_t n2) {
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n2;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    double v = parts[i];
-    for (int c = 1; c < nparts; ++c) v += parts[c * n2 + i];
-    K[i] = v;
-  }
-}
-
-}  // namespace
-
-// The exchange with the half-transform and the SYRK pipelined over `chunks` ranges of aux indices: the
-// main stream half-transforms range c + 1 while the handle's second compute stream runs the SYRK of
-// range c into its own partial K_c; K = sum_c K_c in a fixed order.  Needs the m16 half-transform's
-// operands (even n and pitch, 16-byte aligned Ct).
-void exchange_pipelined(rr_ri_store* h, const double* Ct, int64_t nocc, double* K, cudaStream_t s, int chunks) {
-  const int64_t n = h->n, naux = h->naux, n2 = n * n;
-  auto& c = h->ctx;
-  h->T.ensure(static_cast<size_t>(naux * nocc * n));
-  h->kpart.ensure(static_cast<size_t>(chunks * n2));
-  std::vector<GemmDesc> sk(chunks);
-  std::vector<int64_t> p0(chunks + 1);
-  int64_t want = 1;
-  for (int ci = 0; ci <= chunks; ++ci) p0[ci] = naux * ci / chunks;
-  for (int ci = 0; ci < chunks; ++ci) {
-    GemmDesc& g = sk[ci];
-    g.M = n; g.N = n; g.K = (p0[ci + 1] - p0[ci]) * nocc;
-    g.A = h->T.p + p0[ci] * nocc * n; g.lda = n; g.opA = Op::T;
-    g.B = g.A; g.ldb = n; g.opB = Op::N;
-    g.C = h->kpart.p + ci * n2; g.ldc = n;
-    g.mirror = 1;
-    want = std::max(want, gemm_work_doubles(g));
-  }
-  h->work.ensure(static_cast<size_t>(want));
-  for (int ci = 0; ci < chunks; ++ci) {
-    RR_REQUIRE(half_transform_m16(Ct, nocc, h->B[0].p + p0[ci] * h->pitch[0], h->pitch[0], p0[ci + 1] - p0[ci], n,
-                                  h->T.p + p0[ci] * nocc * n, s, half_transform_config()),
-               RR_ERR_STATE, "exchange_pipelined: operands not supported by the m16 half-transform");
-    RR_CUDA(cudaEventRecord(c.pipe_ev[ci], s));
-    RR_CUDA(cudaStreamWaitEvent(c.pipe_stream, c.pipe_ev[ci], 0));
-    gemm(sk[ci], c.pipe_stream, h->work.p, static_cast<int64_t>(h->work.n));
-  }
-  prof_mark(h, 2, s);
-  RR_CUDA(cudaEventRecord(c.pipe_ev[chunks], c.pipe_stream));
-  RR_CUDA(cudaStreamWaitEvent(s, c.pipe_ev[chunks], 0));
-  sum_parts_kernel<<<static_cast<int>(std::min<int64_t>((n2 + 255) / 256, 1184)), 256, 0, s>>>(K, h->kpart.p, chunks,
-                                                                                               n2);
-  RR_LAUNCH_CHECK();
-}
-
 // Exchange K' = sum_P (Ct B^P)^T (Ct B^P) for a given Ct (nocc x n, row-major with leading
 // dimension ldct, or its transpose when ct_transposed: Ct = C^T with C stored n x nocc).
 // With Dp given (the SCF loop's FP64 build), the Coulomb matrix J of the pitched density Dp is
@@ -123,21 +70,6 @@ void exchange_nonrel(rr_ri_store* h, const double* Ct, int64_t ldct, bool ct_tra
   ht.B = h->B[0].p; ht.ldb = n; ht.opB = Op::N; ht.strideB = h->pitch[0];
   ht.C = h->T.p; ht.ldc = n; ht.strideC = nocc * n;
   ht.batch = naux;
-  // RR_HT_PIPELINE=<chunks> (2 .. 8, for measurement): the drop-in build's half-transform and SYRK
-  // pipelined over that many ranges of aux indices (exchange_pipelined).  Both are DMMA-bound, so running
-  // them side by side gains nothing and the smaller per-chunk SYRKs cost: at n = 400, naux = 1600,
-  // nocc = 40, 1.609 / 1.627 / 1.672 / 1.723 ms per build with 2 / 3 / 4 / 6 chunks against 1.566 ms.
-  static const int pipe_chunks = [] {
-    const char* e = std::getenv("RR_HT_PIPELINE");
-    const int k = e ? std::atoi(e) : 0;
-    return k >= 2 && k <= Context::kPipeMax ? k : 0;
-  }();
-  auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
-  if (pipe_chunks && !Dp && !half_only && K && !ct_transposed && ldct == n && half_transform_kind() == 1 &&
-      n % 2 == 0 && h->pitch[0] % 2 == 0 && al16(Ct) && naux >= 8 * pipe_chunks) {
-    exchange_pipelined(h, Ct, nocc, K, s, pipe_chunks);
-    return;
-  }
   double* tgam = nullptr;
   int tseg = 0;
   if (Dp) {
@@ -446,13 +378,8 @@ void fock_nonrel(rr_ri_store* h, const double* hc, const double* D, const double
     return k >= 1 && k <= 4 ? k : 0;
   }();
   const int j_ctas = j_env ? j_env : static_cast<double>(h->naux) * static_cast<double>(n2) >= 1e8 ? 2 : 1;
-  // RR_J_AFTER_RECOVERY=1 (device pointers, for measurement): the J passes start after the recovery instead.
-  static const bool j_late = [] {
-    const char* e = std::getenv("RR_J_AFTER_RECOVERY");
-    return e && std::atoi(e) == 1;
-  }();
   cudaEvent_t j_from = nullptr;
-  if (!host && !j_late) {  // the J passes wait for what s holds now, not for the recovery that may be queued before them
+  if (!host) {  // the J passes wait for what s holds now, not for the recovery that may be queued before them
     RR_CUDA(cudaEventRecord(h->ctx.upl[0], s));
     j_from = h->ctx.upl[0];
   }
@@ -463,12 +390,11 @@ void fock_nonrel(rr_ri_store* h, const double* hc, const double* D, const double
       copy_in(hd, hc, n2, true, c.side);  // read only by the final combine
       RR_CUDA(cudaEventRecord(c.upl[2], c.side));
       h_ready = c.upl[2];
-    } else if (j_from) {
+    } else {
       RR_CUDA(cudaStreamWaitEvent(c.side, j_from, 0));
       coulomb_early(h, Dp, J, c.side, j_ctas);
     }
   });
-  if (!host && j_late) coulomb_early(h, Dp, J, s, j_ctas);
   if (d_ready) RR_CUDA(cudaStreamWaitEvent(s, d_ready, 0));  // (n_eff = 0 skips the products)
   prof_mark(h, 1, s);
   exchange_nonrel(h, Ct, n, false, nocc, K, s);

@@ -112,15 +112,10 @@ struct Context {
   bool own_main = false;
   cudaEvent_t fork = nullptr, join = nullptr, mid = nullptr;
   cudaEvent_t upl[3] = {nullptr, nullptr, nullptr};  // host-input uploads on the side stream
-  // Second compute stream and its events: the exchange SYRK of one chunk of aux indices runs there
-  // while the main stream half-transforms the next chunk.
-  static constexpr int kPipeMax = 8;
-  cudaStream_t pipe_stream = nullptr;
-  cudaEvent_t pipe_ev[kPipeMax + 1] = {};
   cusolverDnHandle_t solver = nullptr;
   DevBuf<double> solver_work;
   DevBuf<int> solver_info;
-  // fock: with the side and pipe streams, the events and the cuSOLVER handle of the Fock builds and SCF loops.
+  // fock: with the side stream, the events and the cuSOLVER handle of the Fock builds and SCF loops.
   // Contexts of MO tensors and orbital optimisers run on the main stream alone, and most never solve an eigenproblem:
   // solver_handle() makes theirs on first use (cusolverDnCreate and Destroy take 2.7 + 2.4 ms).
   void init(cudaStream_t user_stream, bool fock = true);
