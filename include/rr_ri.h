@@ -43,7 +43,14 @@ extern "C" {
 #define RR_MEM_HOST 0
 #define RR_MEM_DEVICE 1
 
-#define RR_PREC_FP64 0  /* every contraction in FP64 (DMMA tensor cores); matches the reference to ~1e-12 */
+/* RR_PREC_FP64: FP64 in and out, errors of the size FP64 arithmetic leaves; matches the reference to ~1e-12.  J, the recovery, the
+ * functional stage and small exchanges run in FP64 (DMMA tensor cores).  Larger exchanges and MO transforms run on the INT8
+ * tensor cores, on 64-bit integers relative to the largest element of a row.  Their errors are bounded normwise,
+ *   |dK_ab| <~ 2^-48 sqrt(K_aa K_bb),   |dB_mo[P][i][j]| <~ 2^-53 max_a ||B^P_a||_2 ||c_i||_2 ||c_j||_2,
+ * not element by element: an element of K or B_mo that is many orders of magnitude below these has fewer correct digits than
+ * FP64 sums of its own (equally small) terms would give it.  Energies and densities do not see that; a caller that screens by
+ * or divides by such elements asks for rr_ri_set_fp64_products(h, RR_FP64_DMMA). */
+#define RR_PREC_FP64 0
 #define RR_PREC_MIXED 1 /* exchange contractions in split-BF16 (3 products, FP32 accumulate) on tcgen05 */
 
 typedef struct rr_ri_store* rr_ri_handle;
@@ -52,7 +59,7 @@ typedef struct rr_ri_store* rr_ri_handle;
 typedef struct rr_timings {
   double total_ms;          /* first to last event of the call, main stream */
   double recovery_ms;       /* occupied-orbital recovery: GEMMs + eigensolver (+ host readback) */
-  double half_transform_ms; /* T[P] = C_occ^T B^P (batched FP64 DMMA, or split-BF16 tcgen05) */
+  double half_transform_ms; /* T[P] = C_occ^T B^P (INT8 digit planes, FP64 DMMA or split-BF16 tcgen05) */
   double exchange_ms;       /* K = sum_P T[P]^T T[P] (SYRK + split-K reduction) */
   double coulomb_ms;        /* J passes on the side stream (overlaps the exchange) */
   double epilogue_ms;       /* F assembly and output copies */
@@ -91,6 +98,13 @@ int rr_ri_create_4c(const double* B_LL, const double* B_SS, int64_t naux, int64_
                     rr_ri_handle* out);
 
 int rr_ri_destroy(rr_ri_handle h);
+
+/* How the handle's RR_PREC_FP64 calls form their exchange and MO transforms: RR_FP64_DIGITS (default; see RR_PREC_FP64), or
+ * RR_FP64_DMMA, sums of FP64 products throughout (Fock builds of n >= 200 1.5 - 2.9 times, MO transforms 2.3 - 3.7 times slower), which also keeps
+ * no digit copy of the tensor.  Between calls on the handle; not after one of them was captured into a graph that is still used. */
+#define RR_FP64_DIGITS 0
+#define RR_FP64_DMMA 1
+int rr_ri_set_fp64_products(rr_ri_handle h, int32_t products);
 
 /* ---------------- one-time set-up on the device ---------------- */
 

@@ -12,6 +12,7 @@ LIB_PATH = Path(__file__).resolve().parent / "librr_ri.so"
 RR_OK, RR_ERR_ARG, RR_ERR_CUDA, RR_ERR_SOLVER, RR_ERR_TIMEOUT, RR_ERR_NOMEM, RR_ERR_STATE, RR_ERR_UNSUPPORTED = range(8)
 RR_MEM_HOST, RR_MEM_DEVICE = 0, 1
 RR_PREC_FP64, RR_PREC_MIXED = 0, 1
+RR_FP64_DIGITS, RR_FP64_DMMA = 0, 1
 RR_MO_NONREL_SPIN, RR_MO_COMPLEX = 0, 1
 
 _i64 = ctypes.c_int64
@@ -177,6 +178,7 @@ _SIGS = {
     "rr_test_sp2_workspace": (ctypes.c_int, [_i64, _i32, ctypes.POINTER(_i64), ctypes.POINTER(_i64)]),
     "rr_test_ritz": (ctypes.c_int, [_vp, _vp, _i32, _vp]),
     "rr_test_boys": (ctypes.c_int, [_vp, _i64, _i32, _vp]),
+    "rr_ri_set_fp64_products": (ctypes.c_int, [_vp, _i32]),
     "rr_ri_info": (ctypes.c_int, [_vp, ctypes.POINTER(_i64), ctypes.POINTER(_i64), ctypes.POINTER(_i64)]),
     "rr_ri_sync": (ctypes.c_int, [_vp]),
     "rr_ri_fock_nonrel": (ctypes.c_int, [_vp, _vp, _vp, _vp, _vp, _i64, _vp, ctypes.POINTER(Opts)]),

@@ -203,6 +203,22 @@ int rr_ri_destroy(rr_ri_handle h) {
   });
 }
 
+int rr_ri_set_fp64_products(rr_ri_handle h, int32_t products) {
+  return api([&] {
+    auto* s = checked(h);
+    RR_REQUIRE(products == RR_FP64_DIGITS || products == RR_FP64_DMMA, RR_ERR_ARG, "rr_ri_set_fp64_products: unknown kind");
+    s->oz_off = products == RR_FP64_DMMA;
+    std::lock_guard<std::mutex> lock(s->oz_mu);
+    if (!s->oz_off || s->oz_users > 0 || s->oz_pinned) return;
+    for (auto& z : s->oz) {
+      z.planes = nullptr;
+      z.buf.release();
+      z.stats.release();
+      z.made = z.ok = false;
+    }
+  });
+}
+
 int rr_ri_info(rr_ri_handle h, int64_t* naux, int64_t* n, int64_t* ns) {
   return api([&] {
     if (!h) throw rr::Error(RR_ERR_ARG, "null handle");

@@ -239,6 +239,10 @@ bool release_idle_planes(int device) noexcept {
 }
 
 OzUse::OzUse(rr_ri_store* h, cudaStream_t s) : h_(h) {
+  if (h->oz_off) {
+    h_ = nullptr;
+    return;
+  }
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   RR_CUDA(cudaStreamIsCapturing(s, &capture));
   const bool captured = capture != cudaStreamCaptureStatusNone;
@@ -262,6 +266,7 @@ OzUse::OzUse(rr_ri_store* h, cudaStream_t s) : h_(h) {
 }
 
 OzUse::~OzUse() {
+  if (!h_) return;
   std::lock_guard<std::mutex> lock(h_->oz_mu);
   --h_->oz_users;
 }

@@ -35,6 +35,7 @@ struct rr_ri_store {
   std::mutex oz_making, oz_mu;  // oz_mu: the two below, and planes that are given back
   int oz_users = 0;             // calls that are queueing products on the planes
   bool oz_pinned = false;       // a captured graph reads the planes: they stay
+  bool oz_off = false;          // rr_ri_set_fp64_products(RR_FP64_DMMA)
   rr::DevBuf<uint8_t> ozbuf;  // digit planes, exponents and partial sums of one exchange
   // Scratch, grown on demand and reused across calls.
   rr::DevBuf<double> mats;  // per-call matrices (inputs, outputs, intermediates)

@@ -78,6 +78,10 @@ class RiStore:
             self.n, self.ns = nl, ns
         self.naux = naux
 
+    def set_fp64_products(self, kind: str):
+        """"digits" (default) or "dmma": how FP64 calls form the exchange and MO transforms (rr_ri_set_fp64_products)."""
+        L.check(L.lib().rr_ri_set_fp64_products(self.handle, {"digits": L.RR_FP64_DIGITS, "dmma": L.RR_FP64_DMMA}[kind]))
+
     def close(self):
         if self.handle and self.handle.value:
             L.lib().rr_ri_destroy(self.handle)
