@@ -9,11 +9,13 @@
 // warps drain TMEM into FP64 registers (eight INT32 anti-diagonals -> two INT64 -> one double), free it for the
 // next tile's MMAs, then scale and store: FP64, or the digit planes of the result for the next product.
 //
-// Bound: the tensor pipe together with the shared-memory port.  The MMAs of a 128 x 64 x 32 step alone take 1207
-// cycles (7817 INT8 MAC per cycle and SM); with the copies' writes to the same port about 1500.  Measured against
-// the DMMA kernels: n = 400, naux = 1600, nocc = 40: half-transform 773 -> 484 us (2.1 GB of planes read, 4.4 TB/s),
-// SYRK 443 -> 199 us; four components nl = 200, ns = 600, naux = 1000, 40 spinors: half-transforms 5.7 -> 2.7 ms,
-// exchange blocks 15.2 -> 4.9 ms; MO transform n = 400, naux = 1600: 16.9 -> 7.3 ms.
+// Bound, more than one column tile: the tensor pipe as these MMAs drive it.  A step of 128 x 64 x 32 takes 1668 cycles, with
+// the copies and without them (clock64 around 508 steps of 144 tiles): 5660 INT8 MAC per cycle and SM of the nominal 8192 (1152 cycles),
+// 3.3 P operations/s on 148 SMs at 1965 MHz, where cuBLAS' INT8 GEMM of 8192^3 reaches 3.0; divided by the 36 plane pairs, 91 TF/s of
+// FP64 products.  Half-transforms of one column tile (up to 64 orbitals) stream the tensor's planes at 4.4 TB/s and are bound by that.  Against
+// the DMMA kernels: n = 400, naux = 1600, nocc = 40: half-transform 773 -> 484 us (2.1 GB of planes read), SYRK 443 -> 199 us; four
+// components nl = 200, ns = 600, naux = 1000, 40 spinors: half-transforms 5.7 -> 2.7 ms, exchange blocks 15.2 -> 4.9 ms; MO transform
+// n = 400, naux = 1600: 16.9 -> 7.3 ms.
 //
 // digitize_columns_kernel: the three-centre tensor to digit planes, one pass over HBM (the tile of 32 columns
 // stays in shared memory between the search for its largest magnitudes and the conversion).
