@@ -845,7 +845,8 @@ __device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
 // Bound: the launch where no row is concerned, the latency of the fragments for a few rows, the FP64 pipe for all of them.
 // J and K of n = 400, naux = 1600, 40 orbitals with 0 / 1 / 10 / 100 / 399 such rows: 1.01 / 1.15 / 1.16 / 1.98 / 4.45 ms; four
 // components nl = 200, ns = 600, naux = 1000, 40 spinors, 0 / 1 / 10 / 300 of a flavour: 8.1 / 8.6 / 8.7 / 18.3 ms.  Fock builds without
-// such rows: two launches more, 1129 -> 1133 us (n = 400), 1933 -> 1936 us (X2C nl = 200).
+// such rows, two launches more and the sums in the half-transform's epilogue: 1080 -> 1092 us (n = 400), 1925 -> 1929 us (X2C nl = 200),
+// 10251 -> 10288 us (four components).
 template <int PHASE, int PARTS>
 __global__ void __launch_bounds__(32 * kRefitWarps, 2) refit_kernel(const __grid_constant__ RefitArgs g) {
   constexpr int MT = PARTS == 1 ? 5 : 3, SETS = PARTS == 1 ? 1 : 4;

@@ -7,8 +7,10 @@
 
 namespace rr {
 
-// Largest n the one-launch purification takes.  SCF loop, product + step launches / one launch, ms: n = 48 6.4 / 2.7, 160 6.9 /
-// 5.0, 240 9.2 / 7.1, 400 16.5 / 14.8; complex n = 232 4.0 / 3.3, 314 5.1 / 4.2.  Beyond that a step's products fill the GPU by themselves.
+// Largest n the one-launch purification takes.  An iteration of an SCF loop (naux = n / 2), product + step launches / one launch, ms: real n =
+// 240 0.96 / 0.63, 400 1.64 / 1.13, 512 2.01 / 1.53, 640 3.30 / 2.84, 800 5.34 / 5.32; complex n = 232 1.10 / 0.83, 320 1.37 / 1.01,
+// 400 1.58 / 1.43, 512 2.13 / 1.89, 640 4.41 / 4.62.  The two meet near n = 800 and complex 580, where a step's products fill the GPU by
+// themselves; the limits keep clear of that.
 constexpr int64_t kSp2MaxReal = 512, kSp2MaxComplex = 400;
 
 // CTAs of the SCF loops' two-stage reductions.
