@@ -46,7 +46,7 @@ extern "C" {
 /* RR_PREC_FP64: FP64 in and out, errors of the size FP64 arithmetic leaves; matches the reference to ~1e-12.  J, the recovery, the
  * functional stage and small exchanges run in FP64 (DMMA tensor cores).  Larger exchanges and MO transforms run on the INT8
  * tensor cores, on 64-bit integers relative to the largest element of a row.  Their errors are bounded normwise,
- *   |dK_ab| <~ 2^-48 sqrt(K_aa K_bb),   |dB_mo[P][i][j]| <~ 2^-53 max_a ||B^P_a||_2 ||c_i||_2 ||c_j||_2,
+ *   |dK_ab| <~ 2^-47 sqrt(K_aa K_bb),   |dB_mo[P][i][j]| <~ 2^-53 max_a ||B^P_a||_2 ||c_i||_2 ||c_j||_2,
  * not element by element: an element of K or B_mo that is many orders of magnitude below these has fewer correct digits than
  * FP64 sums of its own (equally small) terms would give it.  Energies and densities do not see that; a caller that screens by
  * or divides by such elements asks for rr_ri_set_fp64_products(h, RR_FP64_DMMA). */

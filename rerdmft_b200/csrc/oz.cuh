@@ -10,7 +10,9 @@
 // The 36 plane pairs with i + j <= 7 are kept.  Dropped: the rounding of v, 2^-64 of 2^e, and the pairs of
 // weight 256^6 and below, for K terms of unrelated operands about sqrt(7 K) 74^2 2^-78 of 2^(ex + ey).  Where
 // an operand meets itself (the diagonal of a symmetric product) the pair (4, 4) does not average out: its sum
-// of squares is formed beside the digits (HalfOut::sq) and added by the caller.
+// of squares is formed beside the digits (HalfOut::sq) and added by the caller.  Rows of different functions that coincide beyond
+// digit 4 (equal functions) keep it, kk 74^2 2^-78 of 2^(ea + eb): J and K of 128 functions, equal in pairs, kk = 25600, off by 2^-49.0 of
+// sqrt(K_aa K_bb) at most, against 2^-49.8 on DMMA; of 128 different ones 2^-50.5 against 2^-49.9.
 // INT32 holds 8 K 2^14 for K <= kOzMaxK.
 #pragma once
 
