@@ -87,7 +87,9 @@ int rr_version(void);
  * RR_MEM_DEVICE for B.  The handle binds to the current CUDA device.  When every B^P is symmetric
  * to a few ulps and there is room (at most half of the free device memory), the handle also keeps
  * the packed upper triangles (naux * n(n+1)/2 doubles) for the Coulomb passes, which then stream
- * half of B; otherwise J streams B itself. */
+ * half of B; otherwise J streams B itself.  The first FP64 exchange or MO transform that runs on the INT8 tensor
+ * cores adds digit planes of B (8 bytes an element) while they fit in a quarter of the free memory, and blocks until
+ * they are made; an allocation of the library that fails takes them back. */
 int rr_ri_create(const double* B, int64_t naux, int64_t n, int32_t mem, rr_ri_handle* out);
 
 /* 4-component variant: eri3_LL (naux, nl*nl) and eri3_SS (naux, ns*ns) sharing the aux index
